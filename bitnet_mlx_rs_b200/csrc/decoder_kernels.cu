@@ -397,11 +397,13 @@ __global__ void __launch_bounds__(128) attention_decode_kernel(const AttnParams 
 // by cp.async into a swizzled shared-memory tile, double buffered per warp.  The cache is the 16-row operand of both
 // products (mma.sync.m16n8k16, bf16 in, fp32 out) and the query heads are the 8 columns: S^T[16 positions x 8] = K Q^T and
 // O^T[16 dims x 8] += V^T P^T.  q and the probabilities are fp32, so each goes in as two bf16 terms (x = hi + lo, the
-// remainder of the first rounding), which keeps the products at fp32 accuracy; with up to four heads the hi terms are
-// columns 0-3 and the lo terms columns 4-7 of ONE instruction, 16 of them a tile.  (The heads as the 16-row operand took
-// 64 a tile, three quarters of their rows empty, and twice the accumulators: 27.1 us for 64 sequences at context 600, bound
-// by the warps' instructions at 9 warps an SM.)  P goes from its accumulator layout to the B operand by movmatrix.
+// remainder of the first rounding), which keeps the products at fp32 accuracy: 32 instructions a tile, hi and lo in turn into
+// one accumulator.  (The heads as the 16-row operand took 64 a tile and twice the accumulators: 28.8 us against 24.5 for 64
+// sequences at contexts of 512 to 639, 20/5 heads.)  P goes from its accumulator layout to the B operand by movmatrix.
 // Running maximum and sum per head as in the scalar kernel; the end of the CTA is shared with it.
+// The order of every sum is fixed, because the next projection quantises the outputs again and a last bit moves codes: hi
+// before lo in each k step, and a tile's probabilities as ((p[2t] + p[2t+1]) + p[8+2t]) + p[9+2t] for t = 0..3, then
+// t 0 + 1 and 2 + 3, then these two.
 constexpr int ATC_TILE = 16;                       // positions per tile
 constexpr int ATC_TILE_BYTES = ATC_TILE * 256;     // one of K or V, head_dim 128 in bf16
 
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
 {
     constexpr int HD = 128;
     constexpr float NEG_INF = -3.0e38f;
-    static_assert(G >= 1 && G <= 8, "query heads per KV head sit in rows 0..7 of the operand");
+    static_assert(G >= 1 && G <= 8, "query heads per KV head are the 8 columns of the operand");
 
     extern __shared__ __align__(128) unsigned char atc_smem[];   // [warp][buffer][K tile, V tile]
     __shared__ float s_m[4][8], s_l[4][8];
@@ -476,24 +478,17 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
         __syncthreads();
     }
 
-    // the query heads, scaled, as B-operand fragments, column g: with up to four heads column g < 4 is head g's hi term and
-    // column 4 + h head h's lo term (columns without a head are zero); with eight there is an operand for each term
-    constexpr bool SPLIT_COLS = G <= 4;
-    constexpr int NQ = SPLIT_COLS ? 1 : 2;
-    unsigned q[NQ][8][2];
+    // the query heads, scaled, as B-operand fragments: column g = head g (columns without a head are zero), two bf16 terms each
+    unsigned qhi[8][2], qlo[8][2];
     {
-        const int head = SPLIT_COLS ? (g & 3) : g;
-        const float *qrow = p.qkv + (size_t)b * p.ldq + (size_t)(kvh * G + (head < G ? head : 0)) * HD;
+        const float *qrow = p.qkv + (size_t)b * p.ldq + (size_t)(kvh * G + (g < G ? g : 0)) * HD;
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int d = ks * 16 + h * 8 + 2 * tig;
-                const float x0 = head < G ? qrow[d] * p.scale : 0.0f, x1 = head < G ? qrow[d + 1] * p.scale : 0.0f;
-                unsigned hi, lo;
-                atc_split(x0, x1, hi, lo);
-                if constexpr (SPLIT_COLS) q[0][ks][h] = g < 4 ? hi : lo;
-                else { q[0][ks][h] = hi; q[NQ - 1][ks][h] = lo; }
+                const float x0 = g < G ? qrow[d] * p.scale : 0.0f, x1 = g < G ? qrow[d + 1] * p.scale : 0.0f;
+                atc_split(x0, x1, qhi[ks][h], qlo[ks][h]);
             }
     }
 
@@ -518,8 +513,7 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    // this lane's columns 2 tig and 2 tig + 1 belong to heads h0 and h0 + 1
-    const int h0 = SPLIT_COLS ? 2 * (tig & 1) : 2 * tig;
+    // this lane's columns are heads 2 tig and 2 tig + 1
     float m_run[2] = {NEG_INF, NEG_INF}, l_run[2] = {0.0f, 0.0f};
     float o[8][4];                               // [16-dim tile][fragment register]: dims g, g + 8; this lane's two columns
 #pragma unroll
@@ -546,14 +540,10 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
             const int row = (lmat & 1) * 8 + lrow, c = ks * 2 + (lmat >> 1);
             unsigned ka[4];
             atc_ldmatrix(ka, kt + (unsigned)row * 256 + (unsigned)((c ^ (row & 7)) * 16));
-#pragma unroll
-            for (int t = 0; t < NQ; ++t) atc_mma(sc, ka[0], ka[1], ka[2], ka[3], q[t][ks][0], q[t][ks][1]);
+            atc_mma(sc, ka[0], ka[1], ka[2], ka[3], qhi[ks][0], qhi[ks][1]);
+            atc_mma(sc, ka[0], ka[1], ka[2], ka[3], qlo[ks][0], qlo[ks][1]);
         }
-        if constexpr (SPLIT_COLS) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) sc[r] += __shfl_xor_sync(0xffffffffu, sc[r], 2);   // hi and lo terms
-        }
-        // registers 2 r, 2 r + 1: position base + g + 8 r, heads h0, h0 + 1
+        // registers 2 r, 2 r + 1: position base + g + 8 r, heads 2 tig, 2 tig + 1
         const int base = p0 + tile * ATC_TILE;
         float corr[2], pr[2][2];
 #pragma unroll
@@ -568,25 +558,25 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
             for (int of = 4; of < 32; of <<= 1) tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, of));
             const float m_new = fmaxf(m_run[e], tmax);    // the tile's first position always exists: finite
             corr[e] = m_run[e] > NEG_INF ? expf(m_run[e] - m_new) : 0.0f;
-            float psum = 0.0f;
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                pr[r][e] = sc[2 * r + e] > NEG_INF ? expf(sc[2 * r + e] - m_new) : 0.0f;
-                psum += pr[r][e];
-            }
-#pragma unroll
-            for (int of = 4; of < 32; of <<= 1) psum += __shfl_xor_sync(0xffffffffu, psum, of);
+            for (int r = 0; r < 2; ++r) pr[r][e] = sc[2 * r + e] > NEG_INF ? expf(sc[2 * r + e] - m_new) : 0.0f;
+            // (p[2t] + p[2t+1] + p[8+2t]) + p[9+2t] in the lanes of both positions of pair t
+            const float next = __shfl_xor_sync(0xffffffffu, pr[0][e], 4), next8 = __shfl_xor_sync(0xffffffffu, pr[1][e], 4);
+            float psum = (pr[0][e] + next) + ((g & 1) ? next8 : pr[1][e]);
+            psum += (g & 1) ? pr[1][e] : next8;
+            psum += __shfl_xor_sync(0xffffffffu, psum, 8);
+            psum += __shfl_xor_sync(0xffffffffu, psum, 16);
             l_run[e] = l_run[e] * corr[e] + psum;
             m_run[e] = m_new;
         }
-        // P^T as the B operand of the second product: k = position, column = head (and term)
-        unsigned pb[NQ][2];
+        // P^T as the B operand of the second product: k = position, column = head
+        unsigned phi[2], plo[2];
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             unsigned hi, lo;
             atc_split(pr[r][0], pr[r][1], hi, lo);
-            if constexpr (SPLIT_COLS) pb[0][r] = atc_transpose(tig < 2 ? hi : lo);
-            else { pb[0][r] = atc_transpose(hi); pb[NQ - 1][r] = atc_transpose(lo); }
+            phi[r] = atc_transpose(hi);
+            plo[r] = atc_transpose(lo);
         }
 
         // ---- O = O * corr + P V ----
@@ -598,30 +588,24 @@ __global__ void __launch_bounds__(128, 3) attention_decode_tc_kernel(const AttnP
             atc_ldmatrix_trans(va, vt + (unsigned)row * 256 + (unsigned)((c ^ (row & 7)) * 16));
             o[mt][0] *= corr[0]; o[mt][1] *= corr[1];
             o[mt][2] *= corr[0]; o[mt][3] *= corr[1];
-#pragma unroll
-            for (int t = 0; t < NQ; ++t) atc_mma(o[mt], va[0], va[1], va[2], va[3], pb[t][0], pb[t][1]);
+            atc_mma(o[mt], va[0], va[1], va[2], va[3], phi[0], phi[1]);
+            atc_mma(o[mt], va[0], va[1], va[2], va[3], plo[0], plo[1]);
         }
         __syncwarp();   // every lane is through with this buffer before the next fetch overwrites it
     }
 
     // the four warps' partial results meet in shared memory
-    if constexpr (SPLIT_COLS) {
 #pragma unroll
-        for (int mt = 0; mt < 8; ++mt)
+    for (int e = 0; e < 2; ++e) {
+        const int head = 2 * tig + e;
+        if (head < G) {
+            if (g == 0) { s_m[warp][head] = m_run[e]; s_l[warp][head] = l_run[e]; }
 #pragma unroll
-            for (int r = 0; r < 4; ++r) o[mt][r] += __shfl_xor_sync(0xffffffffu, o[mt][r], 2);   // hi and lo terms
-    }
-    if (!SPLIT_COLS || tig < 2) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-            if (h0 + e < G) {
-                if (g == 0) { s_m[warp][h0 + e] = m_run[e]; s_l[warp][h0 + e] = l_run[e]; }
-#pragma unroll
-                for (int mt = 0; mt < 8; ++mt) {
-                    s_o[warp][h0 + e][mt * 16 + g] = o[mt][e];
-                    s_o[warp][h0 + e][mt * 16 + g + 8] = o[mt][2 + e];
-                }
+            for (int mt = 0; mt < 8; ++mt) {
+                s_o[warp][head][mt * 16 + g] = o[mt][e];
+                s_o[warp][head][mt * 16 + g + 8] = o[mt][2 + e];
             }
+        }
     }
     __syncthreads();
     attention_fold<G, HD>(p, split, kvh, b, tid, s_m, s_l, s_o, &s_last);

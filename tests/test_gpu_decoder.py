@@ -4,6 +4,8 @@ Integer stages (int8 activations, int32 accumulators, the fp32 outputs derived f
 bit for bit, given the fp32 row that the glue in front of them produced on the GPU; floating-point
 stages (SubLN, attention, softmax sums) are compared with the tolerances written below: their sums run
 in another order than the oracle's float64 evaluation."""
+import zlib
+
 import numpy as np
 import pytest
 import torch
@@ -151,6 +153,20 @@ def test_attention_decode_tensor_core_form(n_heads, n_kv, n_splits):
         others = np.arange(max_seq) != pos[b]
         assert np.array_equal(after_k[b][:, others], kc[b][:, others])
     assert ops.device_error_flags() == 0
+
+
+@pytest.mark.parametrize("G,crc", [(1, 0x0169deea), (2, 0x5b6320f4), (4, 0x45f0525a), (8, 0x5a8ace8d)])
+def test_attention_decode_tensor_core_form_keeps_the_order_of_its_sums(G, crc):
+    """The next projection quantises the attention output again, where a last bit moves int8 codes (and a whole model's logits
+    by 3 % of their norm): every bit is pinned, as CRC-32 of the outputs.  The values were computed on a B200 by the kernel's
+    form with the query heads as the 16-row operand, which adds in the same order."""
+    rng = np.random.default_rng(100 + G)
+    qkv = rng.standard_normal((65, (G + 2) * 128)).astype(np.float32)
+    k, v = (dev(rng.standard_normal((65, 1, 200, 128)).astype(np.float32)).bfloat16() for _ in range(2))
+    pos = rng.integers(0, 200, size=65)
+    pos[:6] = [0, 1, 15, 16, 47, 199]
+    out = ops.attention_decode(dev(qkv), k, v, dev(pos.astype(np.int32)), G, 1, 128, n_splits=1)
+    assert zlib.crc32(out.cpu().numpy().tobytes()) == crc
 
 
 def test_sampler_argmax_and_draws():
