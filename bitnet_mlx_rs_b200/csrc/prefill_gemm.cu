@@ -1197,11 +1197,14 @@ bitnet_status_t launch_prefill(const ForwardArgs &a, void *workspace, size_t wor
     const bool pair = a.wp2 != nullptr;
     const PfPlan plan = pf_plan(a.M, a.K, a.N, pair);
     const int n_counters = plan.whole_tiles ? 0 : 2 * (int)plan.tiles;   // only split tiles are counted
+    // The GEMM fetches its weights before it waits for the quantiser.  Rows that the launch in front of the quantiser copied
+    // are there by then only if the quantiser itself started after that launch: no programmatic start behind a copy.
+    const uint32_t q_flags = repack ? a.flags & ~BITNET_FLAG_PDL : a.flags;
     if (a.pre) {   // residual add and normalisation ride in the quantiser
         RowsOut rows = {};
         rows.q_perm = q_perm; rows.pitch = pitch; rows.rowsum = rowsum; rows.a_scale = a_scale;
         rows.counters = counters; rows.n_counters = n_counters;
-        BITNET_TRY(launch_quantize_rows_glued(a.x, a.M, a.K, a.pre, rows, a.q_out, a.a_scale_out, a.flags, stream));
+        BITNET_TRY(launch_quantize_rows_glued(a.x, a.M, a.K, a.pre, rows, a.q_out, a.a_scale_out, q_flags, stream));
     } else {
         cudaLaunchConfig_t qcfg = {};
         cudaLaunchAttribute qattr[1];
@@ -1210,7 +1213,7 @@ bitnet_status_t launch_prefill(const ForwardArgs &a, void *workspace, size_t wor
         qcfg.blockDim = dim3(short_rows ? 128 : 256);
         qcfg.stream = stream;
         qcfg.attrs = qattr;
-        if (a.flags & BITNET_FLAG_PDL) {   // the caller chains launches: start while the previous kernel drains
+        if (q_flags & BITNET_FLAG_PDL) {   // the caller chains launches: start while the previous kernel drains
             qattr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
             qattr[0].val.programmaticStreamSerializationAllowed = 1;
             qcfg.numAttrs = 1;

@@ -220,6 +220,27 @@ def test_any_width_matches_the_generic_kernel(M, K, N):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,K,N", [(8, 1001, 2100), (40, 1001, 6000), (300, 2577, 3000)])
+@pytest.mark.parametrize("glue", [False, True])
+def test_odd_width_in_a_chain_of_programmatic_launches(M, K, N, glue):
+    """Two matrices take turns on one workspace, every launch with programmatic start: the GEMM must read the rows that its own
+    call copied to slice boundaries, not the other matrix's from the call before."""
+    if glue:
+        K = K // 16 * 16 + 16        # the glue takes multiples of 16; none of these is one of 64
+    g = torch.Generator(device="cuda").manual_seed(N)
+    ws, x = [_weights(g, N, K) for _ in range(2)], torch.randn(M, K, device="cuda", generator=g)
+    row_glue = ops.make_glue(residual=x, norm_weight=torch.ones(K, device="cuda"), norm_bias=torch.zeros(K, device="cuda"))
+
+    def call(w, **kw):
+        return ops.bitlinear_forward_fused(w, (N,), (0.02,), x, glue=row_glue, **kw) if glue else ops.bitlinear_forward(w, 0.02, x, N, **kw)
+
+    ref = [call(w, path="generic") for w in ws]
+    out = [call(ws[i % 2], pdl=True) for i in range(20)]
+    assert all(torch.equal(y, ref[i % 2]) for i, y in enumerate(out))
+    assert ops.device_error_flags() == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("K", [1002, 8640])
 def test_any_width_any_alignment_and_workspace(K):
     """Buffers that start anywhere, code 3 (weight 0 to the generic kernel) and a workspace that only suits the generic kernel."""
