@@ -112,3 +112,20 @@ def test_oracle_reproduces_golden_fixtures(path):
     ref = oracle.bitlinear_forward(z["wp"], float(z["w_scale"]), z["x"], int(z["N"]))
     for key in ("q", "acc", "a_scale", "y"):
         assert np.array_equal(ref[key], z[key]), key
+
+
+def test_stack_block_follows_its_values():
+    """Scales may be objects that change between calls (0-d tensors, arrays): the block holds what they hold now."""
+    import torch
+
+    from bitnet_mlx_rs_b200 import ops
+    for cell in (torch.tensor(0.5), np.array(0.5)):
+        assert list(ops._stack([64, 32], [cell, 0.25]).scales) == [0.5, 0.25, 0.0]
+        cell.fill_(9.0) if torch.is_tensor(cell) else cell.fill(9.0)
+        assert list(ops._stack([64, 32], [cell, 0.25]).scales) == [9.0, 0.25, 0.0]
+    st = ops._stack((np.int64(64), torch.tensor(32), 8), (1, np.float32(2.5), -0.0))
+    assert (st.n_members, list(st.rows)) == (3, [64, 32, 8])
+    assert list(st.scales) == [1.0, 2.5, 0.0] and np.signbit(st.scales[2]) and not np.signbit(ops._stack((64, 32, 8), (1, 2.5, 0.0)).scales[2])
+    for rows, scales in (([64.0], [1.0]), ([64], ["1"]), ([1, 2, 3, 4], [1.0])):
+        with pytest.raises((TypeError, IndexError)):
+            ops._stack(rows, scales)
