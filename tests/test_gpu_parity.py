@@ -534,3 +534,37 @@ def test_ffn_throughput_flag_same_bits():
         a, _ = ops.ffn_forward(dev(wg), sg, dev(wu), su, dev(wd), sd, dev(x), 6912)
         b, _ = ops.ffn_forward(dev(wg), sg, dev(wu), su, dev(wd), sd, dev(x), 6912, throughput=True)
         assert torch.equal(a, b)
+
+
+def test_scratch_belongs_to_the_stream_that_uses_it():
+    """Calls on a side stream while the current one is busy: their scratch is neither filled in the current stream's order nor,
+    when it grows, given back to a pool whose next user does not wait for them."""
+    side = torch.cuda.Stream()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    B, kv, G, hd, n_splits = 3, 2, 2, 128, 4
+    qkv = torch.randn(B, (G + 2) * kv * hd, device="cuda", generator=g)
+    k, v = (torch.randn(B, kv, 300, hd, device="cuda", generator=g).bfloat16() for _ in range(2))
+    pos = torch.tensor([299, 7, 140], dtype=torch.int32, device="cuda")
+    ref = ops.attention_decode(qkv, k, v, pos, G * kv, kv, hd, n_splits=n_splits)
+    shapes = [(3, 1001, 700), (40, 1001, 700), (40, 1001, 9000), (200, 3001, 9000)]     # each needs more scratch than the one before
+    calls = []
+    for M, K, N in shapes:
+        w = torch.randint(0, 256, ((N * K + 3) // 4,), dtype=torch.uint8, device="cuda", generator=g)
+        ops.sanitize_packed(w)
+        x = torch.randn(M, K, device="cuda", generator=g)
+        calls.append((w, x, N, ops.bitlinear_forward(w, 0.02, x, N, path="generic"), torch.empty(M, N, device="cuda")))
+    dirty = torch.full((1 << 26,), 255, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    del dirty                                       # the current stream's pool holds memory that is not zero
+    torch.cuda._sleep(50_000_000)                   # 25 ms: nothing queued on the current stream runs before the calls below
+    att = ops.attention_decode(qkv, k, v, pos, G * kv, kv, hd, n_splits=n_splits, stream=side)
+    for w, x, N, _, y in calls:
+        ops.bitlinear_forward(w, 0.02, x, N, out=y, stream=side)
+        for size in (1 << 16, 1 << 20, 1 << 23, 1 << 25):
+            torch.full((size,), 170, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    assert torch.equal(att, ref)
+    for _, _, _, want, y in calls:
+        assert torch.equal(y, want)
+    # the grown buffer comes from the side stream's pool
+    assert any(seg["stream"] == side.cuda_stream for seg in torch.cuda.memory_snapshot())
