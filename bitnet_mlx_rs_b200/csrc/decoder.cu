@@ -285,10 +285,11 @@ extern "C" bitnet_status_t bitnet_decoder_create(bitnet_backend *b, const bitnet
     A(B * F * 4, reinterpret_cast<void **>(&d->h));
     A(B * H * 4, reinterpret_cast<void **>(&d->f));
     A(B * V * 4, reinterpret_cast<void **>(&d->logits));
-    // one workspace for every projection of a step (they run one after the other on one stream)
-    // (the tensor-core path's need grows with the token count, the decode path's peaks at 16 tokens)
+    // one workspace for every projection of a step (they run one after the other on one stream), for every batch up to
+    // max_batch: the need falls where a kernel family that fuses more takes over (hidden 8320 above 8 tokens, which still have
+    // gate and up buffers), and grows with the batch from 129 on
     size_t need = 0, w = 0;
-    for (size_t mm : {B, B > 16 ? (size_t)16 : B}) {
+    for (size_t mm = 1; mm <= B; mm = mm < 129 || mm == B ? mm + 1 : B) {
         if (st == BITNET_OK) st = bitnet_bitlinear_fused_workspace_size(mm, H, QD + 2 * KD, BITNET_PATH_AUTO, &w);
         if (w > need) need = w;
         if (st == BITNET_OK) st = bitnet_bitlinear_fused_workspace_size(mm, QD, H, BITNET_PATH_AUTO, &w);

@@ -271,6 +271,24 @@ def test_decoder_steps_match_the_oracle_model(graphs, max_batch):
         b.close()
 
 
+@pytest.mark.parametrize("max_batch", [9, 16, 24])
+def test_every_batch_up_to_the_largest_runs(max_batch):
+    """Wide layers: up to 8 tokens gate and up go through buffers of their own, which larger batches do not need."""
+    cfg, emb, ls, head = small_model(max_batch=max_batch, H=8320, F=1024)
+    b = cuda.CudaBackend(cuda.CudaBackendConfig(memory_pool_size=1 << 30))
+    try:
+        p = build_pipeline(b, cfg, emb, ls, head)
+        for B in [1, 2, 3, 5, 8, 9, max_batch]:
+            p.reset()
+            p.feed(np.full((B, 2), 7, dtype=np.int32))
+            _, steps = p.decode(np.full(B, 3, dtype=np.int32), 1, SamplingConfig(deterministic=True))
+            assert steps == 1 and np.isfinite(p.logits(B)).all(), B
+        p.close()
+        assert ops.device_error_flags() == 0
+    finally:
+        b.close()
+
+
 def test_generate_stops_at_eos_and_is_reproducible():
     cfg, emb, ls, head = small_model(seed=3, max_batch=4)
     b = cuda.CudaBackend(cuda.CudaBackendConfig(memory_pool_size=1 << 30))
