@@ -59,6 +59,7 @@ public:
         auto it = live_.find(p);
         if (it == live_.end()) return fail(BITNET_ERR_INVALID_CONFIG, "free: pointer was not allocated by this backend");
         allocated_ -= it->second;
+        ++releases_;
         live_.erase(it);
         return check_cuda(cudaFree(p), "cudaFree");
     }
@@ -70,12 +71,23 @@ public:
     size_t pool_size() const { return pool_size_; }
     size_t peak() const { return peak_; }
     uint64_t allocation_count() const { return count_; }
+    // whether the pool would hold `bytes` more once a buffer of `given_back` bytes is released
+    bool has_room(size_t bytes, size_t given_back)
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        return allocated_ - given_back + bytes <= pool_size_;
+    }
+    uint64_t releases()
+    {
+        std::lock_guard<std::mutex> lock(mu_);
+        return releases_;
+    }
 
 private:
     std::mutex mu_;
     size_t pool_size_;
     size_t allocated_ = 0, peak_ = 0;
-    uint64_t count_ = 0;
+    uint64_t count_ = 0, releases_ = 0;
     std::unordered_map<void *, size_t> live_;
 };
 
@@ -87,6 +99,8 @@ struct CudaStream {
     size_t pinned_bytes = 0;
     void *dev = nullptr;      // device staging (x, h, y) + workspace, grown on demand
     size_t dev_bytes = 0;
+    size_t denied_bytes = 0;        // a size that the device had no room for, and the pool's releases by then
+    uint64_t denied_releases = 0;
     std::mutex mu;            // one host-facing call at a time per stream
     // result of an asynchronous host-buffer call that is still in flight on this stream:
     // `pending_bytes` bytes at `pending_src` (pinned staging) go to `pending_dst` once the stream is idle
@@ -161,6 +175,27 @@ public:
             s.dev_bytes = dev_bytes;
         }
         return BITNET_OK;
+    }
+
+    // Staging of `fixed` bytes with a workspace behind it: `want` bytes for the fastest kernel, or `least` for a slower one that
+    // fits.  Whether `want` fits is known before the buffer at hand is given up, so that a call which has to make do with
+    // `least` neither frees nor allocates once it has that much.
+    bitnet_status_t ensure_scratch(CudaStream &s, size_t host_bytes, size_t fixed, size_t want, size_t least, size_t *ws)
+    {
+        *ws = want;
+        if (fixed + want > s.dev_bytes && least < want) {
+            const bool denied = s.denied_bytes && fixed + want >= s.denied_bytes && memory->releases() == s.denied_releases;
+            if (denied || !memory->has_room(fixed + want, s.dev_bytes)) {
+                *ws = least;
+            } else if (ensure_staging(s, host_bytes, fixed + want) != BITNET_OK) {   // the device has less room than the pool
+                *ws = least;
+                const bitnet_status_t st = ensure_staging(s, host_bytes, fixed + least);
+                s.denied_bytes = fixed + want;
+                s.denied_releases = memory->releases();
+                return st;
+            }
+        }
+        return ensure_staging(s, host_bytes, fixed + *ws);
     }
 
     void record(uint64_t ns, uint64_t bytes)
@@ -500,10 +535,7 @@ extern "C" bitnet_status_t bitnet_backend_bitlinear_forward(bitnet_backend *b, c
     BITNET_CUDA(cudaSetDevice(b->impl.device));
     size_t ws = 0;
     BITNET_TRY(bitnet_bitlinear_workspace_size(M, w->impl.K, w->impl.N, opts ? opts->path : BITNET_PATH_AUTO, &ws));
-    if (b->impl.ensure_staging(*s, 0, ws) != BITNET_OK) {   // a pool too small for the fastest kernel's scratch
-        ws = forward_workspace_least(M, w->impl.K, w->impl.N, opts ? opts->path : BITNET_PATH_AUTO);
-        BITNET_TRY(b->impl.ensure_staging(*s, 0, ws));
-    }
+    BITNET_TRY(b->impl.ensure_scratch(*s, 0, 0, ws, forward_workspace_least(M, w->impl.K, w->impl.N, opts ? opts->path : BITNET_PATH_AUTO), &ws));
     const uint64_t t0 = now_ns();
     BITNET_TRY(bitnet_bitlinear_forward(w->impl.packed_dev, w->impl.w_scale, x_dev, y_dev, M, w->impl.K, w->impl.N, opts,
                                         ws ? s->dev : nullptr, ws, s->stream));
@@ -530,10 +562,7 @@ extern "C" bitnet_status_t bitnet_backend_bitlinear_forward_host(bitnet_backend 
     const size_t xb = align_up(M * K * sizeof(float), 256), yb = align_up(M * N * sizeof(float), 256);
     size_t ws = 0;
     BITNET_TRY(bitnet_bitlinear_workspace_size(M, K, N, opts ? opts->path : BITNET_PATH_AUTO, &ws));
-    if (b->impl.ensure_staging(*s, xb + yb, xb + yb + ws) != BITNET_OK) {
-        ws = forward_workspace_least(M, K, N, opts ? opts->path : BITNET_PATH_AUTO);
-        BITNET_TRY(b->impl.ensure_staging(*s, xb + yb, xb + yb + ws));
-    }
+    BITNET_TRY(b->impl.ensure_scratch(*s, xb + yb, xb + yb, ws, forward_workspace_least(M, K, N, opts ? opts->path : BITNET_PATH_AUTO), &ws));
     char *pin = static_cast<char *>(s->pinned), *dev = static_cast<char *>(s->dev);
     const uint64_t t0 = now_ns();
     memcpy(pin, x_host, M * K * sizeof(float));
@@ -573,10 +602,7 @@ static bitnet_status_t ffn_forward_host_common(bitnet_backend *b, const bitnet_w
     const size_t xb = align_up(M * hidden * sizeof(float), 256), hb = align_up(M * ffn * sizeof(float), 256);
     size_t ws = 0;
     BITNET_TRY(bitnet_ffn_workspace_size(M, hidden, ffn, opts ? opts->path : BITNET_PATH_AUTO, &ws));
-    if (b->impl.ensure_staging(*s, 2 * xb, 2 * xb + hb + ws) != BITNET_OK) {
-        ws = ffn_workspace_least(M, hidden, ffn, opts ? opts->path : BITNET_PATH_AUTO);
-        BITNET_TRY(b->impl.ensure_staging(*s, 2 * xb, 2 * xb + hb + ws));
-    }
+    BITNET_TRY(b->impl.ensure_scratch(*s, 2 * xb, 2 * xb + hb, ws, ffn_workspace_least(M, hidden, ffn, opts ? opts->path : BITNET_PATH_AUTO), &ws));
     char *pin = static_cast<char *>(s->pinned), *dev = static_cast<char *>(s->dev);
     float *x_dev = reinterpret_cast<float *>(dev), *y_dev = reinterpret_cast<float *>(dev + xb);
     float *h_dev = reinterpret_cast<float *>(dev + 2 * xb);

@@ -568,3 +568,35 @@ def test_scratch_belongs_to_the_stream_that_uses_it():
         assert torch.equal(y, want)
     # the grown buffer comes from the side stream's pool
     assert any(seg["stream"] == side.cuda_stream for seg in torch.cuda.memory_snapshot())
+
+
+@pytest.mark.parametrize("tight", [True, False])
+def test_backend_pool_without_room_for_the_fastest_scratch(tight):
+    """An odd width in a pool that holds the generic kernel's scratch but not the repacked rows: right, and from the second call on
+    without an allocation (a cudaFree would wait for the busy stream)."""
+    import time
+    M, K, N = 8, 1001, 6000
+    wp, ws, x = case(23, M, K, N)
+    up = lambda n: (n + 255) // 256 * 256   # noqa: E731
+    generic = up(M * K) + up(4 * M)
+    pool = up((N * K + 3) // 4) + 256 + (generic + 4096 if tight else 1 << 24)
+    b = cuda.CudaBackend(cuda.CudaBackendConfig(memory_pool_size=pool, num_streams=1))
+    try:
+        w = b.upload_packed(wp, N, K, ws)
+        dx, y = dev(x), torch.empty(M, N, device="cuda")
+        b.bitlinear_forward(w, dx, y)
+        b.synchronize()
+        ref = ops.bitlinear_forward(dev(wp), ws, dx, N, path="generic")
+        assert torch.equal(y, ref)
+        y.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.ExternalStream(b.stream(0))):
+            torch.cuda._sleep(400_000_000)          # 0.2 s
+        t0 = time.perf_counter()
+        b.bitlinear_forward(w, dx, y)
+        assert time.perf_counter() - t0 < 0.1
+        b.synchronize()
+        assert torch.equal(y, ref)
+        w.free()
+    finally:
+        b.close()
