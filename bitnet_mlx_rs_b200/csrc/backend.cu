@@ -71,11 +71,13 @@ public:
     size_t pool_size() const { return pool_size_; }
     size_t peak() const { return peak_; }
     uint64_t allocation_count() const { return count_; }
-    // whether the pool would hold `bytes` more once a buffer of `given_back` bytes is released
-    bool has_room(size_t bytes, size_t given_back)
+    // Whether `want` bytes may be taken in the place of a buffer of `given_back` bytes where `least` would do: the difference
+    // is scratch for speed (a copy of a whole matrix for an odd width), which leaves three quarters of the pool's room to
+    // what its owner allocates later.
+    bool has_room(size_t want, size_t least, size_t given_back)
     {
         std::lock_guard<std::mutex> lock(mu_);
-        return allocated_ - given_back + bytes <= pool_size_;
+        return allocated_ - given_back + least + 4 * (want - least) <= pool_size_;
     }
     uint64_t releases()
     {
@@ -185,7 +187,7 @@ public:
         *ws = want;
         if (fixed + want > s.dev_bytes && least < want) {
             const bool denied = s.denied_bytes && fixed + want >= s.denied_bytes && memory->releases() == s.denied_releases;
-            if (denied || !memory->has_room(fixed + want, s.dev_bytes)) {
+            if (denied || !memory->has_room(fixed + want, fixed + least, s.dev_bytes)) {
                 *ws = least;
             } else if (ensure_staging(s, host_bytes, fixed + want) != BITNET_OK) {   // the device has less room than the pool
                 *ws = least;
@@ -960,13 +962,15 @@ extern "C" bitnet_status_t bitnet_backend_ffn_plan_create(bitnet_backend *b, con
         pin_bytes += (c.x_pinned ? 0 : xb) + (c.y_pinned ? 0 : xb);
         p->bytes_per_run += 3 * (ffn * hidden / 4) + 4 * c.M * (2 * hidden + 2 * ffn) + 4 * c.M * (2 * ffn + hidden);
     }
-    if (st == BITNET_OK && b->impl.memory->allocate(dev_bytes, &p->dev_slab) != BITNET_OK) {
-        for (PlanCall &c : p->calls) {   // a pool too small for the fastest kernels' scratch
-            dev_bytes -= align_up(c.ws_bytes, 256);
-            c.ws_bytes = ffn_workspace_least(c.M, c.gate->K, c.gate->N, p->opts.path);
-            dev_bytes += align_up(c.ws_bytes, 256);
+    if (st == BITNET_OK) {
+        size_t least = dev_bytes;
+        for (const PlanCall &c : p->calls)
+            least = least - align_up(c.ws_bytes, 256) + align_up(ffn_workspace_least(c.M, c.gate->K, c.gate->N, p->opts.path), 256);
+        if (!b->impl.memory->has_room(dev_bytes, least, 0) || b->impl.memory->allocate(dev_bytes, &p->dev_slab) != BITNET_OK) {
+            // a pool too small for the fastest kernels' scratch
+            for (PlanCall &c : p->calls) c.ws_bytes = ffn_workspace_least(c.M, c.gate->K, c.gate->N, p->opts.path);
+            st = b->impl.memory->allocate(least, &p->dev_slab);
         }
-        st = b->impl.memory->allocate(dev_bytes, &p->dev_slab);
     }
     if (st == BITNET_OK && pin_bytes) st = check_cuda(cudaMallocHost(&p->pin_slab, pin_bytes), "cudaMallocHost");
     if (st == BITNET_OK) {

@@ -600,3 +600,45 @@ def test_backend_pool_without_room_for_the_fastest_scratch(tight):
         w.free()
     finally:
         b.close()
+
+
+def test_backend_scratch_leaves_room_for_later_allocations():
+    """Scratch that only makes an odd width faster takes at most a quarter of the pool's room."""
+    M, K, N = 8, 1001, 6000
+    wp, ws, x = case(23, M, K, N)
+    packed = ((N * K + 3) // 4 + 255) // 256 * 256
+    b = cuda.CudaBackend(cuda.CudaBackendConfig(memory_pool_size=3 * packed, num_streams=2))
+    try:
+        w = b.upload_packed(wp, N, K, ws)
+        y = b.bitlinear_forward_host(w, x)                  # a copy of the rows would take more than one matrix of the two left
+        w2 = b.upload_packed(wp, N, K, ws)
+        assert np.array_equal(b.bitlinear_forward_host(w2, x, stream_idx=1), y)
+        ref = ops.bitlinear_forward(dev(wp), ws, dev(x), N, path="generic")
+        assert np.array_equal(y, ref.cpu().numpy())
+        w.free(); w2.free()
+    finally:
+        b.close()
+
+
+@pytest.mark.parametrize("room", ["all", "some", "least"])
+def test_backend_plan_of_odd_widths_in_pools_of_several_sizes(room):
+    hidden, ffn, Ms = 1000, 1001, [3, 20]
+    shapes = [(ffn, hidden), (ffn, hidden), (hidden, ffn)]
+    packs = [oracle.gen_ternary_packed(29, i, n * k) for i, (n, k) in enumerate(shapes)]
+    scales = [oracle.gen_weight_scale(29, i, k) for i, (_, k) in enumerate(shapes)]
+    extra = {"all": 1 << 26, "some": 1 << 21, "least": 1 << 19}[room]
+    b = cuda.CudaBackend(cuda.CudaBackendConfig(memory_pool_size=3 * 251000 + 2048 + extra, num_streams=1))
+    try:
+        w = [b.upload_packed(p, n, k, s) for p, (n, k), s in zip(packs, shapes, scales)]
+        xs = [oracle.gen_activations(29, 50 + i, (M, hidden)) for i, M in enumerate(Ms)]
+        ys = [np.full((M, hidden), np.nan, dtype=np.float32) for M in Ms]
+        plan = b.ffn_plan([(*w, x, y) for x, y in zip(xs, ys)], n_lanes=1)
+        for _ in range(3):
+            plan.run()
+        for x, y in zip(xs, ys):
+            ref, _ = oracle.ffn_forward(packs[0], scales[0], packs[1], scales[1], packs[2], scales[2], x, ffn)
+            assert np.array_equal(y, ref)
+        plan.close()
+        assert ops.device_error_flags() == 0
+    finally:
+        b.close()
