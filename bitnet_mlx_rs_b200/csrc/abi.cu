@@ -60,16 +60,17 @@ static size_t quant_workspace_bytes(size_t M, size_t K)
 // (us here / there: 8192x640 15.5 / 11.1 at 32 tokens, 15.2 / 12.1 at 64, 15.4 / 16.4 at 128; 8192x2560 16.2 / 13.5, 16.3 / 15.3,
 // 17.5 / 31.7; 4096x1024 10.6 / 9.2, 10.4 / 11.2; 2560x640 8.9 / 8.8, 8.9 / 10.2; 4096x4096 11.7 / 12.8 at 32).
 // `small`: a call of 2 to 16 tokens may take the persistent GEMM too where the weight-streaming kernel is the slower one
-// (prefill_beats_decode).
+// (prefill_beats_decode).  `odd`: widths that are no multiple of 128 may take it as well; false leaves them to the generic kernel,
+// which needs less scratch.
 constexpr int PATH_REPACK = 100;   // inside this file: the persistent GEMM on rows copied to slice boundaries
 
-static int resolve_path(int path, size_t M, size_t K, size_t N, bool small = false)
+static int resolve_path(int path, size_t M, size_t K, size_t N, bool small = false, bool odd = true)
 {
     if (path != BITNET_PATH_AUTO) return path;
     if (M <= 16 && decode_supports(M, K, N) && !(small && prefill_beats_decode(M, K, N))) return BITNET_PATH_DECODE;
     if (M > 16 && M <= 64 && N <= 2560 && K >= (M <= 32 ? 4096 : 6144) && midm_can_run(M, K, N, false)) return BITNET_PATH_CLUSTER;
-    if (prefill_supports_tail(M, K, N)) return BITNET_PATH_PREFILL;
-    if (repack_pays(M, K, N)) return PATH_REPACK;
+    if (odd ? prefill_supports_tail(M, K, N) : prefill_supports(M, K, N)) return BITNET_PATH_PREFILL;
+    if (odd && repack_pays(M, K, N)) return PATH_REPACK;
     return BITNET_PATH_GENERIC;
 }
 
@@ -427,15 +428,15 @@ static const size_t kAmaxBytes = 256 * 16 * sizeof(unsigned);   // up to 256 CTA
 static int call_path(int path, size_t K) { return path == PATH_REPACK || (path == BITNET_PATH_PREFILL && K % 128) ? (int)BITNET_PATH_AUTO : path; }
 
 // Gate and up share one launch: twice the features of a single layer.
-static int pair_path(int path, size_t M, size_t hidden, size_t ffn)
+static int pair_path(int path, size_t M, size_t hidden, size_t ffn, bool odd)
 {
-    const int p = resolve_path(path, M, hidden, ffn);
+    const int p = resolve_path(path, M, hidden, ffn, false, odd);
     return path == BITNET_PATH_AUTO && p == BITNET_PATH_CLUSTER ? (int)BITNET_PATH_PREFILL : p;
 }
 
-static size_t ffn_workspace(size_t M, size_t hidden, size_t ffn, int path, bool glue)
+static size_t ffn_workspace(size_t M, size_t hidden, size_t ffn, int path, bool glue, bool odd = true)
 {
-    const int p1 = pair_path(path, M, hidden, ffn), p2 = resolve_path(path, M, ffn, hidden);
+    const int p1 = pair_path(path, M, hidden, ffn, odd), p2 = resolve_path(path, M, ffn, hidden, false, odd);
     const size_t w1 = forward_workspace(M, hidden, ffn, call_path(p1, hidden), false, false);
     const size_t w2 = forward_workspace(M, ffn, hidden, call_path(p2, ffn), false, false);
     size_t need = kAmaxBytes + (w1 > w2 ? w1 : w2);
@@ -460,10 +461,7 @@ size_t forward_workspace_least(size_t M, size_t K, size_t N, int path)
 size_t ffn_workspace_least(size_t M, size_t hidden, size_t ffn, int path)
 {
     if (M == 0) return 0;
-    const size_t need = ffn_workspace(M, hidden, ffn, path, false);
-    if (path != BITNET_PATH_AUTO || (hidden % 128 == 0 && ffn % 128 == 0)) return need;
-    const size_t generic = ffn_workspace(M, hidden, ffn, BITNET_PATH_GENERIC, false);
-    return generic < need ? generic : need;
+    return ffn_workspace(M, hidden, ffn, path, false, false);
 }
 }  // namespace bitnet
 
@@ -500,13 +498,15 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
         return fail(BITNET_ERR_INVALID_CONFIG, "%s: per-projection debug outputs are not available", who);
     if (o.path < BITNET_PATH_AUTO || o.path > BITNET_PATH_CLUSTER) return fail(BITNET_ERR_INVALID_CONFIG, "unknown path %d", o.path);
     const bool glue = has_glue(pre);
-    // other widths than multiples of 128 make do with the generic kernel's smaller workspace
+    // a block with a width that is no multiple of 128 makes do with less workspace: that projection, or else all three, on the
+    // generic kernel
     int path = o.path;
-    if (path == BITNET_PATH_AUTO && (hidden % 128 || ffn % 128) && workspace_bytes < ffn_workspace(M, hidden, ffn, path, glue))
+    const bool odd = workspace_bytes >= ffn_workspace(M, hidden, ffn, path, glue);
+    if (path == BITNET_PATH_AUTO && (hidden % 128 || ffn % 128) && workspace_bytes < ffn_workspace(M, hidden, ffn, path, glue, false))
         path = BITNET_PATH_GENERIC;
-    BITNET_TRY(check_workspace(workspace_dev, workspace_bytes, ffn_workspace(M, hidden, ffn, path, glue)));
+    BITNET_TRY(check_workspace(workspace_dev, workspace_bytes, ffn_workspace(M, hidden, ffn, path, glue, odd)));
     cudaStream_t s = as_stream(stream);
-    const int p1 = pair_path(path, M, hidden, ffn), p2 = resolve_path(path, M, ffn, hidden);
+    const int p1 = pair_path(path, M, hidden, ffn, odd), p2 = resolve_path(path, M, ffn, hidden, false, odd);
     const bool pair_aligned = ((reinterpret_cast<uintptr_t>(w_gate_dev) | reinterpret_cast<uintptr_t>(w_up_dev) | reinterpret_cast<uintptr_t>(x_dev)) & 15) == 0;
     char *ws = static_cast<char *>(workspace_dev);
     unsigned *amax = reinterpret_cast<unsigned *>(ws);

@@ -282,3 +282,28 @@ def test_ffn_of_any_width_matches_the_generic_kernels(M, H, F):
     ry, rh = ops.ffn_forward(wg, 0.05, wu, 0.04, wd, 0.03, x, F, path="generic")
     assert torch.equal(h, rh) and torch.equal(y, ry)
     assert ops.device_error_flags() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,H,F", [(40, 192, 320), (4, 2560, 1000), (12, 1001, 2560), (20, 2560, 1000)])
+def test_ffn_of_any_width_in_smaller_workspaces(M, H, F):
+    """The size that AUTO asks for, one byte less, and what the generic kernel needs: the same bits from all."""
+    import ctypes as C
+    from bitnet_mlx_rs_b200 import _lib as L
+    g = torch.Generator(device="cuda").manual_seed(F)
+    wg, wu, wd = _weights(g, F, H), _weights(g, F, H), _weights(g, H, F)
+    x = torch.randn(M, H, device="cuda", generator=g)
+    ry, rh = ops.ffn_forward(wg, 0.05, wu, 0.04, wd, 0.03, x, F, path="generic")
+    lib, size = L.load(), {}
+    for path in (L.PATH_AUTO, L.PATH_GENERIC):
+        n = C.c_size_t()
+        assert lib.bitnet_ffn_workspace_size(M, H, F, path, C.byref(n)) == 0
+        size[path] = n.value
+    ws = torch.empty(max(size.values()) + 256, dtype=torch.uint8, device="cuda")
+    base = (ws.data_ptr() + 255) // 256 * 256
+    for nbytes in (size[L.PATH_AUTO], size[L.PATH_AUTO] - 1, size[L.PATH_GENERIC]):
+        y, h = torch.full_like(x, float("nan")), torch.full((M, F), float("nan"), device="cuda")
+        st = lib.bitnet_ffn_forward(wg.data_ptr(), 0.05, wu.data_ptr(), 0.04, wd.data_ptr(), 0.03, x.data_ptr(), h.data_ptr(), y.data_ptr(),
+                                    M, H, F, None, base, nbytes, torch.cuda.current_stream().cuda_stream)
+        assert st == 0 and torch.equal(h, rh) and torch.equal(y, ry), nbytes
+    assert ops.device_error_flags() == 0
