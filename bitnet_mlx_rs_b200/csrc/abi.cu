@@ -274,8 +274,8 @@ static bitnet_status_t forward_impl(const uint8_t *weights_dev, const size_t *ro
     if (o.path == BITNET_PATH_AUTO && K % 128 && (path == BITNET_PATH_PREFILL || path == PATH_REPACK)) {
         // widths that only the generic kernel takes otherwise: it also takes any alignment and a smaller workspace
         const size_t need = path == PATH_REPACK ? repack_workspace_bytes(M, K, N) : prefill_workspace_bytes(M, K, N);
-        const bool mis = path == BITNET_PATH_PREFILL && ((reinterpret_cast<uintptr_t>(weights_dev) | reinterpret_cast<uintptr_t>(x_dev) |
-                                                          reinterpret_cast<uintptr_t>(o.q_out_dev)) & 15);
+        const uintptr_t in = reinterpret_cast<uintptr_t>(weights_dev) | reinterpret_cast<uintptr_t>(x_dev), q_out = reinterpret_cast<uintptr_t>(o.q_out_dev);
+        const bool mis = path == BITNET_PATH_PREFILL ? ((in | q_out) & 15) : (glue && (q_out & 15));   // what their quantisers ask for
         if (mis || o.n_peers || !workspace_dev || (reinterpret_cast<uintptr_t>(workspace_dev) & 255) || workspace_bytes < need)
             path = BITNET_PATH_GENERIC;
     }

@@ -307,3 +307,26 @@ def test_ffn_of_any_width_in_smaller_workspaces(M, H, F):
                                     M, H, F, None, base, nbytes, torch.cuda.current_stream().cuda_stream)
         assert st == 0 and torch.equal(h, rh) and torch.equal(y, ry), nbytes
     assert ops.device_error_flags() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", [1040, 1088])
+def test_odd_width_with_glue_writes_the_activations_anywhere(K):
+    import ctypes as C
+    from bitnet_mlx_rs_b200 import _lib as L
+    M, N = 20, 3000
+    g = torch.Generator(device="cuda").manual_seed(K)
+    w, x = _weights(g, N, K), torch.randn(M, K, device="cuda", generator=g)
+    glue = ops.make_glue(residual=x)
+    y, dbg = ops.bitlinear_forward_fused(w, (N,), (0.02,), x, glue=glue, debug=True)
+    lib, need = L.load(), C.c_size_t()
+    assert lib.bitnet_bitlinear_fused_workspace_size(M, K, N, L.PATH_AUTO, C.byref(need)) == 0
+    ws = torch.empty(need.value + 256, dtype=torch.uint8, device="cuda")
+    for off in (0, 1, 8):
+        q = torch.full((M * K + 16,), 99, dtype=torch.int8, device="cuda")
+        opts, y2 = L.ForwardOpts(q_out_dev=q.data_ptr() + off), torch.full_like(y, float("nan"))
+        st = lib.bitnet_bitlinear_forward_fused(w.data_ptr(), C.byref(ops._stack((N,), (0.02,))), x.data_ptr(), C.byref(glue), y2.data_ptr(), M, K,
+                                                C.byref(opts), (ws.data_ptr() + 255) // 256 * 256, need.value, torch.cuda.current_stream().cuda_stream)
+        assert st == 0 and torch.equal(y2, y)
+        assert torch.equal(q[off:off + M * K].view(M, K), dbg["q"]) and bool((q[:off] == 99).all()) and bool((q[off + M * K:] == 99).all())
+    assert ops.device_error_flags() == 0
