@@ -423,9 +423,12 @@ extern "C" bitnet_status_t bitnet_bitlinear_forward_fused(const uint8_t *weights
 static size_t ffn_pair_bytes(size_t M, size_t ffn) { return align_up(M * ffn * sizeof(float), 256); }
 static const size_t kAmaxBytes = 256 * 16 * sizeof(unsigned);   // up to 256 CTAs x 16 tokens
 
-// How a projection of a block is asked for: a width that is no multiple of 128 by AUTO, which looks at the buffers' alignment
-// and the workspace before it leaves the generic kernel.
-static int call_path(int path, size_t K) { return path == PATH_REPACK || (path == BITNET_PATH_PREFILL && K % 128) ? (int)BITNET_PATH_AUTO : path; }
+// How a projection of a block is asked for: where AUTO (`asked`) found the persistent GEMM for a width that is no multiple of 128,
+// by AUTO again, which looks at the buffers' alignment and the workspace before it leaves the generic kernel.
+static int call_path(int asked, int path, size_t K)
+{
+    return asked == BITNET_PATH_AUTO && (path == PATH_REPACK || (path == BITNET_PATH_PREFILL && K % 128)) ? (int)BITNET_PATH_AUTO : path;
+}
 
 // Gate and up share one launch: twice the features of a single layer.
 static int pair_path(int path, size_t M, size_t hidden, size_t ffn, bool odd)
@@ -437,10 +440,10 @@ static int pair_path(int path, size_t M, size_t hidden, size_t ffn, bool odd)
 static size_t ffn_workspace(size_t M, size_t hidden, size_t ffn, int path, bool glue, bool odd = true)
 {
     const int p1 = pair_path(path, M, hidden, ffn, odd), p2 = resolve_path(path, M, ffn, hidden, false, odd);
-    const size_t w1 = forward_workspace(M, hidden, ffn, call_path(p1, hidden), false, false);
-    const size_t w2 = forward_workspace(M, ffn, hidden, call_path(p2, ffn), false, false);
+    const size_t w1 = forward_workspace(M, hidden, ffn, call_path(path, p1, hidden), false, false);
+    const size_t w2 = forward_workspace(M, ffn, hidden, call_path(path, p2, ffn), false, false);
     size_t need = kAmaxBytes + (w1 > w2 ? w1 : w2);
-    if ((p1 == BITNET_PATH_PREFILL && call_path(p1, hidden) == p1) || (p1 == BITNET_PATH_CLUSTER && midm_can_run(M, hidden, ffn, true)))
+    if ((p1 == BITNET_PATH_PREFILL && call_path(path, p1, hidden) == p1) || (p1 == BITNET_PATH_CLUSTER && midm_can_run(M, hidden, ffn, true)))
         need += 0;   // the pair launch gates in its epilogue: no gate/up buffers, the glue rides in its quantiser
     else if (p1 != BITNET_PATH_DECODE || !decode_supports_dual(M, hidden, ffn))
         need += 2 * ffn_pair_bytes(M, ffn) + (glue ? glue_bytes(M, hidden) : 0);
@@ -498,6 +501,8 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
         return fail(BITNET_ERR_INVALID_CONFIG, "%s: per-projection debug outputs are not available", who);
     if (o.path < BITNET_PATH_AUTO || o.path > BITNET_PATH_CLUSTER) return fail(BITNET_ERR_INVALID_CONFIG, "unknown path %d", o.path);
     const bool glue = has_glue(pre);
+    if (o.path == BITNET_PATH_PREFILL && (!prefill_supports(M, hidden, ffn) || !prefill_supports(M, ffn, hidden)))
+        return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "%s: prefill kernel does not cover M=%zu hidden=%zu ffn=%zu", who, M, hidden, ffn);
     // a block with a width that is no multiple of 128 makes do with less workspace: that projection, or else all three, on the
     // generic kernel
     int path = o.path;
@@ -515,10 +520,8 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
     const bool fused_pair = p1 == BITNET_PATH_DECODE && decode_supports_dual(M, hidden, ffn);
     // the gate/up launch leaves per-CTA absmax keys of h; the down launch folds them instead of re-reading h
     const bool chain_amax = fused_pair && p2 == BITNET_PATH_DECODE && decode_grid(ffn) <= 256;
-    if ((p1 == BITNET_PATH_PREFILL && (pair_aligned || hidden % 128 == 0)) || (p1 == BITNET_PATH_CLUSTER && midm_can_run(M, hidden, ffn, true))) {
+    if ((p1 == BITNET_PATH_PREFILL && (pair_aligned || call_path(path, p1, hidden) == p1)) || (p1 == BITNET_PATH_CLUSTER && midm_can_run(M, hidden, ffn, true))) {
         // gate and up as the two halves of one launch; its epilogue applies up * relu(gate)^2
-        if (o.path == BITNET_PATH_PREFILL && !prefill_supports(M, hidden, ffn))
-            return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "prefill kernel does not cover M=%zu K=%zu N=%zu", M, hidden, ffn);
         ForwardArgs a = {};
         a.wp = w_gate_dev; a.w_scale = s_gate; a.wp2 = w_up_dev; a.w_scale2 = s_up;
         a.x = x_dev; a.y = h_dev; a.M = M; a.K = hidden; a.N = ffn; a.ldy = ffn; a.flags = o.flags;
@@ -552,7 +555,7 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
             BITNET_TRY(launch_row_pre(x_dev, M, hidden, r, o.flags, s));
         }
         bitnet_forward_opts po = {};
-        po.path = call_path(p1, hidden); po.flags = o.flags;
+        po.path = call_path(path, p1, hidden); po.flags = o.flags;
         BITNET_TRY(bitnet_bitlinear_forward(w_up_dev, s_up, x_eff, up, M, hidden, ffn, &po, ws + off, workspace_bytes - off, stream));
         BITNET_TRY(bitnet_bitlinear_forward(w_gate_dev, s_gate, x_eff, gate, M, hidden, ffn, &po, ws + off, workspace_bytes - off, stream));
         BITNET_TRY(launch_gate_relu2(up, gate, h_dev, M * ffn, s));
@@ -568,7 +571,7 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
         return launch_decode(a, s);
     }
     bitnet_forward_opts po = {};
-    po.path = call_path(p2, ffn); po.flags = o.flags; po.stages = o.stages;
+    po.path = call_path(path, p2, ffn); po.flags = o.flags; po.stages = o.stages;
     return bitnet_bitlinear_forward(w_down_dev, s_down, h_dev, y_dev, M, ffn, hidden, &po, ws + off, workspace_bytes - off, stream);
 }
 

@@ -129,3 +129,14 @@ def test_stack_block_follows_its_values():
     for rows, scales in (([64.0], [1.0]), ([64], ["1"]), ([1, 2, 3, 4], [1.0])):
         with pytest.raises((TypeError, IndexError)):
             ops._stack(rows, scales)
+
+
+@pytest.mark.parametrize("hidden,ffn", [(256, 192), (192, 256), (256, 1000)])
+@pytest.mark.parametrize("M", [4, 40, 200])
+def test_ffn_by_a_named_path_refuses_widths_the_path_does_not_take(M, hidden, ffn):
+    """Refused before anything is launched: the addresses are never used."""
+    lib, opts = L.load(), L.ForwardOpts(path=L.PATH_PREFILL)
+    args = (M, hidden, ffn, C.byref(opts), 1 << 20, 1 << 40, None)
+    for fn, glue in ((lib.bitnet_ffn_forward, ()), (lib.bitnet_ffn_forward_fused, (None,))):
+        st = fn(4096, 0.1, 4096, 0.1, 4096, 0.1, 4096, *glue, 4096, 4096, *args)
+        assert st == L.ERR_UNSUPPORTED_OPERATION, lib.bitnet_last_error_string()
