@@ -281,8 +281,10 @@ static bitnet_status_t forward_impl(const uint8_t *weights_dev, const size_t *ro
     }
     if (o.n_peers < 0 || o.n_peers > BITNET_MAX_PEERS)
         return fail(BITNET_ERR_INVALID_CONFIG, "n_peers must be in 0..%d (got %d)", BITNET_MAX_PEERS, o.n_peers);
-    if (o.n_peers > 0 && o.path == BITNET_PATH_AUTO && M > 16 && M <= 128 && N <= 32768 && midm_can_run(M, K, N, false))
-        return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "peer outputs of 17 to 128 tokens: name the path (prefill)");
+    // AUTO has never written peer outputs for up to 128 tokens of these layers (its kernel there was the cluster GEMM, which
+    // cannot): which GPU's kernel runs must not depend on a routing rule, so the caller names the path
+    if (o.n_peers > 0 && o.path == BITNET_PATH_AUTO && path != BITNET_PATH_DECODE && M <= 128 && N <= 32768 && midm_can_run(M, K, N, false))
+        return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "peer outputs of up to 128 tokens beyond the decode kernel: name the path (prefill)");
     if (o.n_peers > 0 && path != BITNET_PATH_DECODE && !(path == BITNET_PATH_PREFILL && n_members == 1 && !o.acc_out_dev))
         return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "peer outputs are written by the decode kernel (M <= 16) and by the persistent GEMM (path prefill)");
 

@@ -140,3 +140,11 @@ def test_ffn_by_a_named_path_refuses_widths_the_path_does_not_take(M, hidden, ff
     for fn, glue in ((lib.bitnet_ffn_forward, ()), (lib.bitnet_ffn_forward_fused, (None,))):
         st = fn(4096, 0.1, 4096, 0.1, 4096, 0.1, 4096, *glue, 4096, 4096, *args)
         assert st == L.ERR_UNSUPPORTED_OPERATION, lib.bitnet_last_error_string()
+
+
+@pytest.mark.parametrize("M,K,N", [(9, 16384, 256), (16, 8320, 32768), (17, 2560, 640), (128, 2560, 2560)])
+def test_auto_refuses_peer_outputs_where_the_cluster_kernel_was_its_choice(M, K, N):
+    opts = L.ForwardOpts(n_peers=1)
+    opts.y_peers_dev[0] = 4096
+    st = L.load().bitnet_bitlinear_forward(4096, 0.1, 4096, 4096, M, K, N, C.byref(opts), 1 << 20, 1 << 40, None)
+    assert st == L.ERR_UNSUPPORTED_OPERATION

@@ -642,3 +642,12 @@ def test_backend_plan_of_odd_widths_in_pools_of_several_sizes(room):
         assert ops.device_error_flags() == 0
     finally:
         b.close()
+
+
+def test_peer_addresses_as_an_array():
+    M, K, N = 4, 256, 64
+    wp, ws, x = case(31, M, K, N)
+    ref = ops.bitlinear_forward(dev(wp), ws, dev(x), N)
+    outs = [torch.zeros(M, N, device="cuda") for _ in range(2)]
+    ops.bitlinear_forward(dev(wp), ws, dev(x), N, y_peers=np.array([o.data_ptr() for o in outs], dtype=np.uint64))
+    assert all(torch.equal(o, ref) for o in outs)
