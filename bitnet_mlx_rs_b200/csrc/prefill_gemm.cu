@@ -1025,17 +1025,21 @@ static size_t pf_tiles(size_t M, size_t N, int bt, bool pair = false)
     const size_t f = pair ? PF_BF / 2 : PF_BF;
     return ((M + bt - 1) / bt) * ((N + f - 1) / f);
 }
-// Estimated device cycles of a plan, from timings of eleven shapes (16 to 2048 tokens, K 384 to 8192) at every tile and
-// both ways of dealing: a k slice costs what its MMAs take (2.22 clk a token) and never less than 290; finishing a tile
-// costs 1000 per 32 tokens and 700 around it, hidden behind the next tile's MMAs unless K is short, and seen once at the
-// end; splitting tiles between CTAs costs another 4500 + 80 a token, so it pays only when whole tiles leave most of a wave
-// idle (256x8192x28672, 3.03 waves of 128 tokens: 51.6 against 53.1 us; 2048x2560x6912, 4.74 of 160: 48.0 against 37.7).
+// Estimated device cycles of a plan, from timings of 23 shapes (16 to 2048 tokens, K 128 to 8192) at every tile and both ways
+// of dealing: a k slice costs what its MMAs take (2.22 clk a token) and never less than 290; finishing a tile costs what is
+// hidden behind the next tile's MMAs unless K is short (per 32 tokens 1400 and 1700 around it where three expander groups leave
+// the epilogue fewer registers, 1000 and 2500 above 128 tokens; the gate/up pair writes half as much), and is seen once at the
+// end; splitting tiles between CTAs costs another 4500 + 80 a token, so it pays only when whole tiles leave most of a wave idle
+// (256x8192x28672, 3.03 waves of 128 tokens: 49.7 against 52.7 us; 2048x2560x6912, 4.74 of 160: 49.9 against 40.0).  Against one
+// line for all tiles, which took 128 tokens where K is short: 2048x128x20000 69.7 -> 59.0 us, 2048x1024x32768 118.8 -> 100.4,
+// 300x1024x32768 28.5 -> 23.6, 2048x640x5000 27.3 -> 22.9, 512x512x16384 22.3 -> 19.1, 2048x2560x6912 41.7 -> 40.0.
 static double pf_plan_cost(size_t M, size_t K, size_t N, int bt, bool whole, size_t sms, bool pair)
 {
     const double k = (double)((K + PF_BK - 1) / PF_BK), tiles = (double)pf_tiles(M, N, bt, pair);
     const double per_slice = 2.22 * bt > 290.0 ? 2.22 * bt : 290.0;
     const double epilogue = 1000.0 * (bt / 32);
-    const double tile = k * per_slice > epilogue + 700.0 ? k * per_slice : epilogue + 700.0;
+    const double between = pair ? 700.0 + epilogue : (pf_groups(bt) == 2 ? 2500.0 + 1000.0 * (bt / 32) : 1700.0 + 1400.0 * (bt / 32));
+    const double tile = k * per_slice > between ? k * per_slice : between;
     if (tiles <= (double)sms) return k * per_slice + epilogue;
     if (whole) return (double)((size_t)((tiles + sms - 1) / sms)) * tile + epilogue;
     return tiles / (double)sms * tile + epilogue + 4500.0 + 80.0 * bt;
