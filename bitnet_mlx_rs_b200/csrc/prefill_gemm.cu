@@ -1085,8 +1085,10 @@ bool prefill_beats_decode(size_t M, size_t K, size_t N)
     if (M < 2 || M > 16 || !prefill_supports(M, K, N)) return false;
     const size_t sms = (size_t)device_sm_count();
     const double blocks = (double)(((N + 15) / 16 + sms - 1) / sms);
-    const PfPlan pl = pf_plan(M, K, N, false);
-    const double here = 6500.0 + pf_plan_cost(M, K, N, pl.bt, pl.whole_tiles, sms, false) / 1.9;
+    // tiles of 32 tokens in whole waves (pf_plan_cost has the cost between wider tiles; these two estimates are fitted to each other)
+    const double k = (double)(K / PF_BK), tiles = (double)pf_tiles(M, N, 32);
+    const double chain = tiles <= (double)sms ? k * 290.0 : (double)((size_t)((tiles + sms - 1) / sms)) * (k * 290.0 > 1700.0 ? k * 290.0 : 1700.0);
+    const double here = 6500.0 + (chain + 1000.0) / 1.9;
     const double decode = M > 8 ? 6500.0 + blocks * (150.0 + 300.0 * (double)K / 1024.0) : 7000.0 + blocks * (450.0 + 55.0 * (double)K / 1024.0);
     return here * (M > 8 ? 1.05 : 1.25) < decode;
 }
