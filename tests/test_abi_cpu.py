@@ -126,6 +126,8 @@ def test_stack_block_follows_its_values():
     st = ops._stack((np.int64(64), torch.tensor(32), 8), (1, np.float32(2.5), -0.0))
     assert (st.n_members, list(st.rows)) == (3, [64, 32, 8])
     assert list(st.scales) == [1.0, 2.5, 0.0] and np.signbit(st.scales[2]) and not np.signbit(ops._stack((64, 32, 8), (1, 2.5, 0.0)).scales[2])
+    assert list(ops._stack([64], [1e39]).scales)[0] == float("inf") and list(ops._stack([64, 1], [2.0]).scales) == [2.0, 0.0, 0.0]
+    assert C.sizeof(L.Stack) == ops._STACKS[3].size
     for rows, scales in (([64.0], [1.0]), ([64], ["1"]), ([1, 2, 3, 4], [1.0])):
         with pytest.raises((TypeError, IndexError)):
             ops._stack(rows, scales)
