@@ -54,11 +54,9 @@ static size_t quant_workspace_bytes(size_t M, size_t K)
     return align_up(M * K, 256) + align_up(M * sizeof(float), 256);
 }
 
-// Which kernel family AUTO takes.  Above 16 tokens the persistent GEMM (2560x6912: 10.1 against the cluster GEMM's 12.1 us at
-// 32 tokens, 10.7 / 13.7 at 64, 11.7 / 17.1 at 128; 8192x8192 at 64: 17.7 / 29.9), but for few tokens through a long and narrow
-// layer: its tiles are serial chains of k slices (6.5 us and 0.14 a slice) on a handful of SMs, and the cluster GEMM splits K
-// (us here / there: 8192x640 15.5 / 11.1 at 32 tokens, 15.2 / 12.1 at 64, 15.4 / 16.4 at 128; 8192x2560 16.2 / 13.5, 16.3 / 15.3,
-// 17.5 / 31.7; 4096x1024 10.6 / 9.2, 10.4 / 11.2; 2560x640 8.9 / 8.8, 8.9 / 10.2; 4096x4096 11.7 / 12.8 at 32).
+// Which kernel family AUTO takes.  Beyond the weight-streaming kernel the persistent GEMM (2560x6912: 10.1 against the cluster
+// GEMM's 12.1 us at 32 tokens, 10.7 / 13.7 at 64, 11.7 / 17.1 at 128; 8192x8192 at 64: 17.7 / 29.9), but for up to 128 tokens
+// through a long and narrow layer, whose K the cluster GEMM splits (midm_beats_prefill).
 // `small`: a call of 2 to 16 tokens may take the persistent GEMM too where the weight-streaming kernel is the slower one
 // (prefill_beats_decode).  `odd`: widths that are no multiple of 128 may take it as well; false leaves them to the generic kernel,
 // which needs less scratch.
@@ -68,7 +66,7 @@ static int resolve_path(int path, size_t M, size_t K, size_t N, bool small = fal
 {
     if (path != BITNET_PATH_AUTO) return path;
     if (M <= 16 && decode_supports(M, K, N) && !(small && prefill_beats_decode(M, K, N))) return BITNET_PATH_DECODE;
-    if (M > 16 && M <= 64 && N <= 2560 && K >= (M <= 32 ? 4096 : 6144) && midm_can_run(M, K, N, false)) return BITNET_PATH_CLUSTER;
+    if (M <= 128 && midm_beats_prefill(M, K, N)) return BITNET_PATH_CLUSTER;
     if (odd ? prefill_supports_tail(M, K, N) : prefill_supports(M, K, N)) return BITNET_PATH_PREFILL;
     if (odd && repack_pays(M, K, N)) return PATH_REPACK;
     return BITNET_PATH_GENERIC;

@@ -119,6 +119,7 @@ bitnet_status_t prefill_take_error_flags(unsigned *flags);
 // Cluster split-K tensor-core GEMM for a few dozen tokens (midm_gemm.cu).
 bool midm_supports(size_t M, size_t K, size_t N);
 bool midm_can_run(size_t M, size_t K, size_t N, bool pair);
+bool midm_beats_prefill(size_t M, size_t K, size_t N);   // at most 128 tokens: faster than the persistent GEMM
 size_t midm_workspace_bytes(size_t M, size_t K);
 bitnet_status_t launch_midm(const ForwardArgs &a, void *workspace, size_t workspace_bytes, bool ready, cudaStream_t stream);
 bitnet_status_t midm_take_error_flags(unsigned *flags);

@@ -479,6 +479,28 @@ bool midm_can_run(size_t M, size_t K, size_t N, bool pair)
     return midm_supports(M, K, N) && midm_plan(M, K, N, pair, &pl);
 }
 
+// Which of the two tensor-core kernels is the faster one for at most 128 tokens: estimates in ns fitted to 2000 timings of both
+// (graph replay, quantiser included, weights from memory; 9 to 128 tokens, K 1024 to 12288, N 128 to 4096), each within 4 % of
+// nearly all.  The persistent GEMM's tiles are serial chains of k slices on a handful of SMs where N is small; here K is split,
+// and the rows of a wider tile cost more (us here / there: 8192x640 11.2 / 14.7 at 32 tokens, 12.1 / 14.5 at 64, 16.1 / 14.5 at 128;
+// 8192x3072 13.0 / 15.3 at 32, 13.9 / 15.4 at 48; 4096x2560 10.2 / 10.4, 11.1 / 10.4; 12288x2560 14.2 / 20.2 at 12 tokens).
+// Beyond about 200 CTAs the launch falls off a cliff as soon as the quantiser's CTAs (one a token) are in its way: 224 CTAs run
+// at 40 tokens and not at 48 (12288x3584: 17.7, 27.8), 240 at 21 (12288x3840: 17.0, 18.9 at 24), 256 at 18 and not at 20
+// (8192x4096: 13.5, 20.9), and slow down before it (4096x3584: 10.2 at 24 tokens, 11.3 at 30); with one CTA an SM it lies
+// between 112 and 128.  The margin sends ties to the kernel without cliffs.
+bool midm_beats_prefill(size_t M, size_t K, size_t N)
+{
+    MidPlan pl;
+    if (!midm_supports(M, K, N) || !midm_plan(M, K, N, false, &pl)) return false;
+    const bool two = pl.smem <= 110 * 1024;   // CTAs per SM
+    if (two ? pl.ctas > 200 && M > (pl.ctas <= 232 ? 40u : (pl.ctas <= 240 ? 22u : 18u)) : pl.ctas > 112) return false;
+    if (pl.ctas > 256) return false;
+    const double S = (double)(K / MM_BK), ns = (double)((K / MM_BK + pl.ck - 1) / pl.ck);
+    const double here = 4300.0 + 620.0 * ns + 820.0 * (pl.mt / 16) + 1300.0 * (double)pl.ctas / 148.0 + (pl.ctas > 200 && M > 24 ? 900.0 : 0.0);
+    const double there = 6350.0 + 120.0 * S + 7.0 * S * (double)M / 128.0 + 39e-6 * (double)N * (double)K + (M > 96 && N >= 1024 ? 30.0 * S : 0.0);
+    return 1.03 * here < there;
+}
+
 bitnet_status_t tensor_map_2d(void *map_out, const void *base, uint64_t inner, uint64_t rows, uint64_t row_stride_bytes,
                               uint32_t box_inner, uint32_t box_rows, int swizzle_128b);
 
