@@ -529,6 +529,9 @@ decode_kernel(const DecodeParams p)
 // Semantics: TernaryProcessor::quantize_activations (ternary_operations.rs:130-163).
 // pre: the decoder-layer glue in front of the quantiser (residual add, SubLN), applied to the row while it
 // sits in registers; sums run in a fixed order (lane tree, then the sixteen warps in turn).
+// COUNTERS: it also clears rows.counters for the persistent GEMM (a form of its own: the loop, even over none, took 0.1 to 0.2 us
+// of the decode kernel's calls, 1280 -> 768 with glue at 3 tokens 7.58 against 7.73).
+template <bool COUNTERS>
 __global__ void __launch_bounds__(512) decode_quantize_kernel(const float *x, int M, int K, int cw, int sw, int nt, int mrows,
                                                               unsigned char *__restrict__ image,
                                                               const unsigned *__restrict__ amax_in, int n_amax_in,
@@ -538,8 +541,10 @@ __global__ void __launch_bounds__(512) decode_quantize_kernel(const float *x, in
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the decode kernel may start fetching weights
     asm volatile("griddepcontrol.wait;" ::: "memory");
     quantize_row_to_image(x, (int)blockIdx.x, K, cw, sw, nt, mrows, image, amax_in, n_amax_in, q_out, a_scale_out, pre, rows);
-    if (blockIdx.x == 0)
-        for (int i = threadIdx.x; i < rows.n_counters; i += 512) rows.counters[i] = 0u;
+    if constexpr (COUNTERS) {
+        if (blockIdx.x == 0)
+            for (int i = threadIdx.x; i < rows.n_counters; i += 512) rows.counters[i] = 0u;
+    }
 }
 
 // The glue and the quantiser for the tensor-core kernels' many rows (K <= 1024 * WARPS): WARPS warps per token,
@@ -728,8 +733,8 @@ bitnet_status_t launch_quantize_rows_glued(const float *x, size_t M, size_t K, c
         else BITNET_CUDA(cudaLaunchKernelEx(&cfg, glued_rows_kernel<8>, x, (int)K, rp, rows, q_out, a_scale_out));
         return BITNET_OK;
     }
-    BITNET_CUDA(cudaLaunchKernelEx(&cfg, decode_quantize_kernel, x, (int)M, (int)K, 1, 1, 1, 1, static_cast<unsigned char *>(nullptr),
-                                   static_cast<const unsigned *>(nullptr), 0, q_out, a_scale_out, rp, rows));
+    BITNET_CUDA(cudaLaunchKernelEx(&cfg, rows.n_counters ? decode_quantize_kernel<true> : decode_quantize_kernel<false>, x, (int)M, (int)K, 1, 1, 1, 1,
+                                   static_cast<unsigned char *>(nullptr), static_cast<const unsigned *>(nullptr), 0, q_out, a_scale_out, rp, rows));
     return BITNET_OK;
 }
 
@@ -1002,7 +1007,7 @@ bitnet_status_t launch_decode(const ForwardArgs &a, cudaStream_t stream)
             cfg.numAttrs = 1;
         }
         if (!a.image_ready)
-            BITNET_CUDA(cudaLaunchKernelEx(&cfg, decode_quantize_kernel, a.x, (int)a.M, (int)a.K, pl.cw, pl.sw, pl.nt, p.mrows,
+            BITNET_CUDA(cudaLaunchKernelEx(&cfg, decode_quantize_kernel<false>, a.x, (int)a.M, (int)a.K, pl.cw, pl.sw, pl.nt, p.mrows,
                                            static_cast<unsigned char *>(a.image_ws), a.amax_in, a.n_amax_in, a.q_out,
                                            a.a_scale_out, pre, RowsOut{}));
         p.image = static_cast<const unsigned char *>(a.image_ws);
