@@ -142,7 +142,7 @@ def _weights(g, n, k):
 @pytest.mark.parametrize("M,H,F", [
     (17, 128, 132),       # one k slice, the last feature tile nearly empty
     (65, 384, 1000),      # an odd number of slices, both halves on CTAs of their own
-    (200, 256, 20000),    # more tiles than SMs: a CTA meets both halves of a tile, and halves of two tiles
+    (200, 256, 20000),    # more tiles than SMs: a CTA takes several in turn (the pair is never split between CTAs)
     (33, 512, 130),       # rows of h that TMA cannot store (plain stores)
     (700, 2560, 640),
 ])
@@ -152,9 +152,9 @@ def test_gate_up_pair_matches_the_generic_kernels(M, H, F):
     wg, wu, wd = _weights(g, F, H), _weights(g, F, H), _weights(g, H, F)
     x = torch.randn(M, H, device="cuda", generator=g)
     x[M // 2] = 0.0       # an all-zero token
-    for _ in range(2):    # the counters of the tiles start over
+    ry, rh = ops.ffn_forward(wg, 0.05, wu, 0.04, wd, 0.03, x, F, path="generic")
+    for _ in range(2):    # again over what the first call left in the workspace
         y, h = ops.ffn_forward(wg, 0.05, wu, 0.04, wd, 0.03, x, F)
-        ry, rh = ops.ffn_forward(wg, 0.05, wu, 0.04, wd, 0.03, x, F, path="generic")
         assert torch.equal(h, rh) and torch.equal(y, ry)
     assert ops.device_error_flags() == 0
 
@@ -162,7 +162,9 @@ def test_gate_up_pair_matches_the_generic_kernels(M, H, F):
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,K,rows", [(20, 256, (128, 64, 64)), (130, 384, (200, 56, 8)), (300, 1024, (1, 300)), (1000, 2560, (2560, 640, 640)),
                                       (2, 1024, (30000, 3000)), (12, 512, (20000, 10000, 77)),
-                                      (149, 4096, (128, 64, 64)), (150, 5120, (64, 10)), (160, 8192, (128,)), (149, 128, (64,)), (150, 16384, (64,))])
+                                      (149, 4096, (128, 64, 64)), (150, 5120, (64, 10)), (160, 8192, (128,)), (149, 128, (64,)), (150, 16384, (64,)),
+                                      # tiles split between CTAs: both quantisers that clear the tiles' counters
+                                      (200, 8192, (9000, 600, 100)), (140, 8192, (19000,))])
 def test_stacked_members_with_glue_match_the_generic_kernels(M, K, rows):
     g = torch.Generator(device="cuda").manual_seed(M)
     w = _weights(g, sum(rows), K)
@@ -170,7 +172,7 @@ def test_stacked_members_with_glue_match_the_generic_kernels(M, K, rows):
     nw, nb = torch.randn(K, device="cuda", generator=g), torch.randn(K, device="cuda", generator=g)
     scales = [0.05, 0.07, 0.02][:len(rows)]
     out = {}
-    for path in ("auto", "prefill", "generic"):
+    for path in ("generic", "prefill", "auto"):
         s, n = torch.empty_like(x), torch.empty_like(x)
         glue = ops.make_glue(residual=res, sum_out=s, norm_weight=nw, norm_bias=nb, eps=1e-5, normed_out=n)
         y, dbg = ops.bitlinear_forward_fused(w, rows, scales, x, glue=glue, path=path, debug=True)
@@ -182,9 +184,10 @@ def test_stacked_members_with_glue_match_the_generic_kernels(M, K, rows):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,K,N", [(2, 1024, 32768), (8, 2560, 60000), (9, 4096, 11008), (16, 128, 40001)])
+@pytest.mark.parametrize("M,K,N", [(2, 1024, 32768), (9, 4096, 11008), (16, 256, 80001), (8, 128, 60000),     # AUTO leaves the decode kernel
+                                   (8, 2560, 60000), (16, 128, 40001)])                                       # and stays
 def test_small_calls_on_either_kernel(M, K, N):
-    """Shapes at which AUTO leaves the weight-streaming kernel: the same bits from both, and without a workspace."""
+    """Shapes on both sides of the line between the two kernels: the same bits from both, and without a workspace."""
     import ctypes as C
     from bitnet_mlx_rs_b200 import _lib as L
     g = torch.Generator(device="cuda").manual_seed(M)
@@ -206,7 +209,9 @@ def test_small_calls_on_either_kernel(M, K, N):
     (17, 64, 50), (100, 8640, 320), (200, 192, 300), (2048, 320, 130),            # multiples of 64: half of the last slice is empty
     (1, 1001, 2100), (9, 333, 5000), (40, 1000, 600), (130, 130, 5000),           # rows that start in the middle of a byte
     (40, 8192, 640), (32, 4096, 1100), (33, 4096, 1100), (65, 8192, 2560),          # either side of the line to the cluster kernel
-    (33, 4, 40000), (3, 65, 20001), (16, 16400, 140), (300, 2576, 77),            # one slice, one code past a slice, wide, no multiple of 4 rows
+    (33, 4, 40000), (3, 65, 20001), (16, 16400, 140), (300, 2576, 77),            # (short rows stay on the generic kernel), wide, no multiple of 4 rows
+    (700, 4, 4000), (40, 65, 20001), (90, 129, 333), (60, 127, 1001),             # one slice, one code past half a slice, past and short of a slice
+    (200, 8256, 9700), (200, 8200, 9700),                                         # tiles split between CTAs, the last slice partly empty
 ])
 def test_any_width_matches_the_generic_kernel(M, K, N):
     g = torch.Generator(device="cuda").manual_seed(K)
