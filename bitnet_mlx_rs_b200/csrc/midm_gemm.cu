@@ -497,7 +497,7 @@ bool midm_beats_prefill(size_t M, size_t K, size_t N)
     if (pl.ctas > 256) return false;
     const double S = (double)(K / MM_BK), ns = (double)((K / MM_BK + pl.ck - 1) / pl.ck);
     const double here = 4300.0 + 620.0 * ns + 820.0 * (pl.mt / 16) + 1300.0 * (double)pl.ctas / 148.0 + (pl.ctas > 200 && M > 24 ? 900.0 : 0.0);
-    const double there = 6350.0 + 120.0 * S + 7.0 * S * (double)M / 128.0 + 39e-6 * (double)N * (double)K + (M > 96 && N >= 1024 ? 30.0 * S : 0.0);
+    const double there = 6350.0 + 120.0 * S + 7.0 * S * (double)M / 128.0 + 39e-6 * (double)N * (double)K + (M > 96 && N >= 1024 ? 40.0 * S : 0.0);
     return 1.03 * here < there;
 }
 
