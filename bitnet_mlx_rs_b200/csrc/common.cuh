@@ -152,7 +152,7 @@ bitnet_status_t launch_seed_rng(unsigned long long *rng, size_t B, unsigned long
 // One thread of a converged warp, picked by the hardware.  Loops that issue tcgen05 and bulk-copy instructions run under
 // this and not under `lane == 0`: those instructions take their operands from uniform registers, and only for an elected
 // thread does the compiler know that a single thread is active and needs no loop over the lanes around each of them
-// (a tcgen05.mma issued from `lane == 0` took 115 clk of the issuing thread, from an elected thread 62).
+// (a tcgen05.mma of the persistent GEMM takes 78 to 86 clk of the issuing thread from `lane == 0`, 16 to 20 from an elected one).
 __device__ __forceinline__ bool elect_one()
 {
     unsigned p;

@@ -714,8 +714,10 @@ bitnet_status_t launch_attention_decode(const float *qkv, size_t ldq, size_t k_o
         s += align_up(B * n_heads * n_splits * 8, 256);
         p.counters = reinterpret_cast<unsigned *>(s);
     }
-    // the tensor-core form from 64 (sequence, KV head) pairs on; below that its fixed cost per CTA (query fragments,
-    // the first tile's round trip) outweighs the cheaper positions (measured: 14.3 against 12.5 us at 40 pairs)
+    // the tensor-core form from 64 (sequence, KV head) pairs on: against the scalar form 12.7 / 14.7 us at context 640 and
+    // 18.4 / 26.4 at 2000 (64 pairs, 4 heads each); its fixed cost per CTA (query fragments, the first tile's round trip) shows at
+    // short contexts (5.4 / 4.5 at 40) and with few pairs (40 pairs: 10.5 / 10.3 at 200, 11.8 / 12.2 at 640).  From about 40
+    // pairs and 600 keys on it is the faster one too, but the forms round differently: moving the line moves logits
     if (head_dim == 128 && B * n_kv >= 64 && (G == 1 || G == 2 || G == 4 || G == 8)) {
         if (G == 1) return launch_attention_tc<1>(p, B, flags, stream);
         if (G == 2) return launch_attention_tc<2>(p, B, flags, stream);

@@ -21,11 +21,12 @@
 //        4 warps     epilogue: tcgen05.ld the accumulator, subtract the row sum
 //                    (sum_k (code-1) q = sum_k code q - sum_k q), scale, stage 32 x 32 blocks in
 //                    shared memory and write y with TMA stores
-//      What bounds it: at 192 tokens the MMAs (784 clk a pair at the int8 rate; 809 measured); at 128 and fewer the
-//      instructions of the single threads and warps that feed them (a barrier wait costs 90 clk even when the phase is
-//      over, an MMA 14 clk to issue), about 290 clk a slice.  2048x2560x6912 38.0 us = 1909 TOPS with its quantiser (56.0
-//      before the roles were taken apart and their loops run by elected threads), 256x8192x28672 50.8 (88.0),
-//      64x2560x128256 32.8 us (63.1).
+//      What bounds it: above 128 tokens the MMAs (653 clk a pair of slices at the int8 rate with 160 tokens; 745 measured where
+//      k is long); at 128 and fewer the instructions of the single threads and warps that feed them, 565 to 665 clk a
+//      pair.  In the MMA thread (clock reads around each part, five shapes): the wait for the pair 200 to 250, the eight MMAs
+//      130 to 160 (16 to 20 each to issue), commit and ring step 110 to 270.  With its quantiser, weights from memory:
+//      2048x2560x6912 40.0 us = 1813 TOPS (55.9 before the roles were taken apart and their loops run by elected threads),
+//      256x8192x28672 49.7 (86.2), 64x2560x128256 32.5 us (63.1).
 //      Work is dealt in whole tiles, or -- when whole tiles would leave most of a wave idle -- in
 //      equal runs of k slices with an exact integer fix-up of the tiles shared by two CTAs.
 //      Every barrier wait is bounded; a wait that runs out raises an error flag and the CTA
@@ -56,7 +57,8 @@ constexpr int PF_WP_BYTES = PF_BF * PF_BK / 4;     // 4 KB packed
 // Groups of four warps that expand packed weights, working on alternate pairs.  One takes about 1300 clk a pair (its waits
 // 470, masks and shifts 300, the tensor-memory store 350): two keep ahead of the MMAs of a tile above 128 tokens (784 clk a
 // pair at 192), narrower ones take three (64x2560x128256: 36.2 -> 33.7 us; at 192 tokens the smaller register share of the
-// wider CTA makes three the slower choice, 26.3 against 27.8 us for 192x8192x18944).
+// wider CTA makes three the slower choice, 26.3 against 27.8 us for 192x8192x18944).  Three groups are 608 threads of 96
+// registers: 64 bytes of stores and 176 of loads are spilled (gate/up pair 40 and 84; none with two groups).
 constexpr int pf_groups(int bt) { return bt > 128 ? 2 : 3; }
 constexpr int pf_threads(int groups) { return (2 + 4 * groups + 4 + 1) * 32; }   // activation loads, MMA, expanders, epilogue, weight loads
 constexpr unsigned PF_WAIT_LIMIT = 1u << 17;      // tries of at most 16 us each
@@ -618,8 +620,8 @@ prefill_gemm_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_cons
     } else if (warp == 1) {
         // ===================== MMA issuer =====================
         if (elect_one()) {
-            // this thread's instructions bound the whole kernel (an MMA takes it about 40 clk to issue): one wait, one
-            // commit and no index arithmetic beyond two ring steps per pair
+            // this thread's instructions bound the kernel at narrow tiles: one wait, one commit and no index arithmetic beyond
+            // two ring steps per pair
             int xr = 0;
             unsigned x_phase = 0;
             const unsigned tmem_a0 = tmem_base + 2u * (unsigned)p.bt, tmem_a_end = tmem_a0 + (unsigned)(p.aslots * PF_PAIR * PF_A_COLS);
