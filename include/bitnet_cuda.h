@@ -61,9 +61,14 @@ const char *bitnet_last_error_string(void);
 
 /* Which kernel family runs a forward call. */
 enum {
-    BITNET_PATH_AUTO = 0,    /* decode kernel for M <= 16, cluster GEMM up to 128 tokens, persistent GEMM beyond */
+    BITNET_PATH_AUTO = 0,    /* by shape: the decode kernel up to 16 tokens (the persistent GEMM from 2 on where N is large for
+                                its K), the persistent GEMM beyond, the cluster GEMM for up to 128 tokens of long and narrow
+                                layers.  Other widths than multiples of 128 run on the persistent GEMM too (from multiples
+                                of 64 as they are, else from a copy of the rows in the workspace) where that pays, the buffers
+                                are 16-byte aligned and the workspace has the size the query asks for, else on the generic
+                                kernel.  All give the same bits */
     BITNET_PATH_DECODE = 1,  /* weight-streaming GEMV family, M <= 16, K % 64 == 0 */
-    BITNET_PATH_PREFILL = 2, /* TMA + tcgen05 int8 GEMM, K % 128 == 0 */
+    BITNET_PATH_PREFILL = 2, /* persistent TMA + tcgen05 int8 GEMM, K % 128 == 0 (other widths through AUTO) */
     BITNET_PATH_GENERIC = 3, /* any M, K, N (rows may start mid-byte); slow, exact */
     BITNET_PATH_CLUSTER = 4  /* TMA + tcgen05 int8 GEMM with K split over a thread-block cluster, 1 <= M <= 128, K % 128 == 0 */
 };
@@ -143,8 +148,10 @@ void launch_w2a8_gemv_optimized(const uint8_t *weights, const int8_t *activation
  * BitLinearForward::forward_with_quantized_weights (bitnet-quant/src/bitlinear/forward.rs:95)
  * compute for a 2-D input.  The argument order follows the reference's only batched
  * quantised-GEMM signature (bitnet-metal/src/mps/matrix_ops.rs:318-341).
- * workspace_dev: bitnet_bitlinear_workspace_size() bytes, 256-byte aligned; may be NULL
- * when that size is 0 (the decode path needs none). */
+ * workspace_dev: bitnet_bitlinear_workspace_size() bytes, 256-byte aligned; may be NULL when that
+ * size is 0.  With path AUTO the size is what the fastest kernel wants: shapes that the decode
+ * kernel takes run without a workspace as well, and widths that are no multiple of 128 with the
+ * generic kernel's, each more slowly. */
 bitnet_status_t bitnet_bitlinear_forward(const uint8_t *weights_dev, float w_scale,
                                          const float *x_dev, float *y_dev,
                                          size_t M, size_t K, size_t N,
@@ -310,7 +317,8 @@ bitnet_status_t bitnet_quantize_pack_weights_workspace_size(size_t n_values, siz
  * consumes the canonical layout (layout_id 0, the only one accepted) -- so preparation is the
  * in-place removal of code 3 plus the shape checks of the fast paths: *fast_paths receives a mask
  * (bit 0: decode kernel usable for M <= 16, bit 1: tensor-core GEMM usable); shapes that fit
- * neither still run on the generic kernel.  count_dev as in bitnet_sanitize_packed. */
+ * neither still run: on the tensor-core GEMM from a copy of the rows, or on the generic kernel.  count_dev as in
+ * bitnet_sanitize_packed. */
 bitnet_status_t bitnet_prepare_weights(uint8_t *packed_dev, size_t N, size_t K, int32_t layout_id,
                                        unsigned long long *count_dev, uint32_t *fast_paths,
                                        bitnet_stream_t stream);
@@ -395,7 +403,8 @@ bitnet_status_t bitnet_backend_free_weights(bitnet_backend *b, bitnet_weights *w
 bitnet_status_t bitnet_weights_info(const bitnet_weights *w, size_t *N, size_t *K, float *w_scale,
                                     const uint8_t **packed_dev);
 
-/* BitLinear forward on device buffers through the backend (workspace from the pool). */
+/* BitLinear forward on device buffers through the backend (workspace from the pool; scratch that only makes an odd width
+ * faster takes at most a quarter of the room the pool has left). */
 bitnet_status_t bitnet_backend_bitlinear_forward(bitnet_backend *b, const bitnet_weights *w,
                                                  const float *x_dev, float *y_dev, size_t M,
                                                  const bitnet_forward_opts *opts, size_t stream_idx);
