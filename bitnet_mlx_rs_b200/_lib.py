@@ -136,7 +136,7 @@ SIGNATURES = {
     "bitnet_backend_bitlinear_forward_host": (i32, [vp, vp, vp, vp, sz, _P(ForwardOpts), sz]),
     "bitnet_backend_ffn_forward_host": (i32, [vp, vp, vp, vp, vp, vp, sz, _P(ForwardOpts), sz]),
     "bitnet_backend_ffn_forward_host_async": (i32, [vp, vp, vp, vp, vp, vp, sz, _P(ForwardOpts), sz]),
-    "bitnet_bitlinear_forward_fused": (i32, [vp, _P(Stack), vp, _P(RowGlue), vp, sz, sz, _P(ForwardOpts), vp, sz, vp]),
+    "bitnet_bitlinear_forward_fused": (i32, [vp, vp, vp, _P(RowGlue), vp, sz, sz, _P(ForwardOpts), vp, sz, vp]),
     "bitnet_bitlinear_fused_workspace_size": (i32, [sz, sz, sz, i32, _P(sz)]),
     "bitnet_ffn_forward_fused": (i32, [vp, f32, vp, f32, vp, f32, vp, _P(RowGlue), vp, vp, sz, sz, sz, _P(ForwardOpts), vp, sz, vp]),
     "bitnet_ffn_fused_workspace_size": (i32, [sz, sz, sz, i32, _P(sz)]),

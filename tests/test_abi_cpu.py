@@ -119,15 +119,19 @@ def test_stack_block_follows_its_values():
     import torch
 
     from bitnet_mlx_rs_b200 import ops
+
+    def block(rows, scales):
+        return L.Stack.from_buffer_copy(ops._stack(rows, scales))
+
     for cell in (torch.tensor(0.5), np.array(0.5)):
-        assert list(ops._stack([64, 32], [cell, 0.25]).scales) == [0.5, 0.25, 0.0]
+        assert list(block([64, 32], [cell, 0.25]).scales) == [0.5, 0.25, 0.0]
         cell.fill_(9.0) if torch.is_tensor(cell) else cell.fill(9.0)
-        assert list(ops._stack([64, 32], [cell, 0.25]).scales) == [9.0, 0.25, 0.0]
-    st = ops._stack((np.int64(64), torch.tensor(32), 8), (1, np.float32(2.5), -0.0))
+        assert list(block([64, 32], [cell, 0.25]).scales) == [9.0, 0.25, 0.0]
+    st = block((np.int64(64), torch.tensor(32), 8), (1, np.float32(2.5), -0.0))
     assert (st.n_members, list(st.rows)) == (3, [64, 32, 8])
-    assert list(st.scales) == [1.0, 2.5, 0.0] and np.signbit(st.scales[2]) and not np.signbit(ops._stack((64, 32, 8), (1, 2.5, 0.0)).scales[2])
-    assert list(ops._stack([64], [1e39]).scales)[0] == float("inf") and list(ops._stack([64, 1], [2.0]).scales) == [2.0, 0.0, 0.0]
-    assert C.sizeof(L.Stack) == ops._STACKS[3].size
+    assert list(st.scales) == [1.0, 2.5, 0.0] and np.signbit(st.scales[2]) and not np.signbit(block((64, 32, 8), (1, 2.5, 0.0)).scales[2])
+    assert list(block([64], [1e39]).scales)[0] == float("inf") and list(block([64, 1], [2.0]).scales) == [2.0, 0.0, 0.0]
+    assert all(p.size == C.sizeof(L.Stack) for p in ops._STACKS.values())
     for rows, scales in (([64.0], [1.0]), ([64], ["1"]), ([1, 2, 3, 4], [1.0])):
         with pytest.raises((TypeError, IndexError)):
             ops._stack(rows, scales)

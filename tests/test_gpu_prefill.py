@@ -330,7 +330,7 @@ def test_odd_width_with_glue_writes_the_activations_anywhere(K):
     for off in (0, 1, 8):
         q = torch.full((M * K + 16,), 99, dtype=torch.int8, device="cuda")
         opts, y2 = L.ForwardOpts(q_out_dev=q.data_ptr() + off), torch.full_like(y, float("nan"))
-        st = lib.bitnet_bitlinear_forward_fused(w.data_ptr(), C.byref(ops._stack((N,), (0.02,))), x.data_ptr(), C.byref(glue), y2.data_ptr(), M, K,
+        st = lib.bitnet_bitlinear_forward_fused(w.data_ptr(), ops._stack((N,), (0.02,)), x.data_ptr(), C.byref(glue), y2.data_ptr(), M, K,
                                                 C.byref(opts), (ws.data_ptr() + 255) // 256 * 256, need.value, torch.cuda.current_stream().cuda_stream)
         assert st == 0 and torch.equal(y2, y)
         assert torch.equal(q[off:off + M * K].view(M, K), dbg["q"]) and bool((q[:off] == 99).all()) and bool((q[off + M * K:] == 99).all())
