@@ -234,7 +234,8 @@ def test_odd_width_in_a_chain_of_programmatic_launches(M, K, N, glue):
         K = K // 16 * 16 + 16        # the glue takes multiples of 16; none of these is one of 64
     g = torch.Generator(device="cuda").manual_seed(N)
     ws, x = [_weights(g, N, K) for _ in range(2)], torch.randn(M, K, device="cuda", generator=g)
-    row_glue = ops.make_glue(residual=x, norm_weight=torch.ones(K, device="cuda"), norm_bias=torch.zeros(K, device="cuda"))
+    nw, nb = torch.ones(K, device="cuda"), torch.zeros(K, device="cuda")      # (the glue holds addresses, not tensors)
+    row_glue = ops.make_glue(residual=x, norm_weight=nw, norm_bias=nb)
 
     def call(w, **kw):
         return ops.bitlinear_forward_fused(w, (N,), (0.02,), x, glue=row_glue, **kw) if glue else ops.bitlinear_forward(w, 0.02, x, N, **kw)
