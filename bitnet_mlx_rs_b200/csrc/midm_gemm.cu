@@ -487,7 +487,8 @@ bool midm_can_run(size_t M, size_t K, size_t N, bool pair)
 // Beyond about 200 CTAs the launch falls off a cliff as soon as the quantiser's CTAs (one a token) are in its way: 224 CTAs run
 // at 40 tokens and not at 48 (12288x3584: 17.7, 27.8), 240 at 21 (12288x3840: 17.0, 18.9 at 24), 256 at 18 and not at 20
 // (8192x4096: 13.5, 20.9), and slow down before it (4096x3584: 10.2 at 24 tokens, 11.3 at 30); with one CTA an SM it lies
-// between 112 and 128.  The margin sends ties to the kernel without cliffs.
+// between 112 and 128.  The persistent GEMM's slices get slower where four token tiles meet about 130000 outputs (8192x1536:
+// 15.0 us at 96 tokens, 16.3 at 112).  The margin sends ties to the kernel without cliffs.
 bool midm_beats_prefill(size_t M, size_t K, size_t N)
 {
     MidPlan pl;
@@ -497,7 +498,7 @@ bool midm_beats_prefill(size_t M, size_t K, size_t N)
     if (pl.ctas > 256) return false;
     const double S = (double)(K / MM_BK), ns = (double)((K / MM_BK + pl.ck - 1) / pl.ck);
     const double here = 4300.0 + 620.0 * ns + 820.0 * (pl.mt / 16) + 1300.0 * (double)pl.ctas / 148.0 + (pl.ctas > 200 && M > 24 ? 900.0 : 0.0);
-    const double there = 6350.0 + 120.0 * S + 7.0 * S * (double)M / 128.0 + 39e-6 * (double)N * (double)K + (M > 96 && N >= 1024 ? 40.0 * S : 0.0);
+    const double there = 6350.0 + 120.0 * S + 7.0 * S * (double)M / 128.0 + 39e-6 * (double)N * (double)K + (M > 96 && M * N >= 130000 ? 40.0 * S : 0.0);
     return 1.03 * here < there;
 }
 
