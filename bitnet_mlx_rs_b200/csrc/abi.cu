@@ -243,6 +243,13 @@ static RowPre to_row_pre(const bitnet_row_glue *g)
     return r;
 }
 static bool has_glue(const RowPre &r) { return r.residual || r.norm_w; }
+static bool row_pre_fits(const float *x, size_t K, const RowPre &r)
+{
+    uintptr_t all = 0;
+    for (const void *ptr : {(const void *)x, (const void *)r.residual, (const void *)r.sum_out, (const void *)r.norm_w, (const void *)r.norm_b, (const void *)r.normed_out})
+        all |= reinterpret_cast<uintptr_t>(ptr);
+    return K % 16 == 0 && K <= 16384 && (all & 15) == 0;
+}
 
 // The stacked members of a launch: the first takes a.w_scale, the others their own scales from their first row on.
 static void set_members(ForwardArgs &a, const size_t *rows, const float *scales, int n_members)
@@ -273,7 +280,8 @@ static bitnet_status_t forward_impl(const uint8_t *weights_dev, const size_t *ro
         // widths that only the generic kernel takes otherwise: it also takes any alignment and a smaller workspace
         const size_t need = path == PATH_REPACK ? repack_workspace_bytes(M, K, N) : prefill_workspace_bytes(M, K, N);
         const uintptr_t in = reinterpret_cast<uintptr_t>(weights_dev) | reinterpret_cast<uintptr_t>(x_dev), q_out = reinterpret_cast<uintptr_t>(o.q_out_dev);
-        const bool mis = path == BITNET_PATH_PREFILL ? ((in | q_out) & 15) : (glue && (q_out & 15));   // what their quantisers ask for
+        // what their quantisers ask for (glue that no kernel takes is refused by the generic path before anything is launched)
+        const bool mis = path == BITNET_PATH_PREFILL ? ((in | q_out) & 15) != 0 : glue && (!row_pre_fits(x_dev, K, pre) || (q_out & 15));
         if (mis || o.n_peers || !workspace_dev || (reinterpret_cast<uintptr_t>(workspace_dev) & 255) || workspace_bytes < need)
             path = BITNET_PATH_GENERIC;
     }
@@ -503,12 +511,15 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
     const bool glue = has_glue(pre);
     if (o.path == BITNET_PATH_PREFILL && (!prefill_supports(M, hidden, ffn) || !prefill_supports(M, ffn, hidden)))
         return fail(BITNET_ERR_UNSUPPORTED_OPERATION, "%s: prefill kernel does not cover M=%zu hidden=%zu ffn=%zu", who, M, hidden, ffn);
-    // a block with a width that is no multiple of 128 makes do with less workspace: that projection, or else all three, on the
-    // generic kernel
+    // a block with a width that is no multiple of 128 makes do with less workspace: that projection, or else (also where buffers
+    // are not aligned) all three, on the generic kernel
     int path = o.path;
     const bool odd = workspace_bytes >= ffn_workspace(M, hidden, ffn, path, glue);
-    if (path == BITNET_PATH_AUTO && (hidden % 128 || ffn % 128) && workspace_bytes < ffn_workspace(M, hidden, ffn, path, glue, false))
-        path = BITNET_PATH_GENERIC;
+    if (path == BITNET_PATH_AUTO && (hidden % 128 || ffn % 128) && !odd) {
+        const uintptr_t all = reinterpret_cast<uintptr_t>(w_gate_dev) | reinterpret_cast<uintptr_t>(w_up_dev) | reinterpret_cast<uintptr_t>(w_down_dev) |
+                              reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(h_dev);
+        if ((all & 15) || workspace_bytes < ffn_workspace(M, hidden, ffn, path, glue, false)) path = BITNET_PATH_GENERIC;
+    }
     BITNET_TRY(check_workspace(workspace_dev, workspace_bytes, ffn_workspace(M, hidden, ffn, path, glue, odd)));
     cudaStream_t s = as_stream(stream);
     const int p1 = pair_path(path, M, hidden, ffn, odd), p2 = resolve_path(path, M, ffn, hidden, false, odd);

@@ -154,3 +154,14 @@ def test_auto_refuses_peer_outputs_where_the_cluster_kernel_was_its_choice(M, K,
     opts.y_peers_dev[0] = 4096
     st = L.load().bitnet_bitlinear_forward(4096, 0.1, 4096, 4096, M, K, N, C.byref(opts), 1 << 20, 1 << 40, None)
     assert st == L.ERR_UNSUPPORTED_OPERATION
+
+
+@pytest.mark.parametrize("K,off,status", [(1002, 0, "ERR_UNSUPPORTED_OPERATION"), (3000, 0, "ERR_UNSUPPORTED_OPERATION"), (16400, 0, "ERR_UNSUPPORTED_OPERATION"),
+                                          (1040, 4, "ERR_INVALID_CONFIG"), (2576, 1, "ERR_INVALID_CONFIG")])
+def test_glue_that_no_kernel_takes_is_refused_before_anything_runs(K, off, status):
+    """Odd widths with row glue: the addresses are never used."""
+    lib, M, N = L.load(), 40, 3000
+    glue = L.RowGlue(4096 + off, None, None, None, 1e-5, None)
+    stack = L.Stack(1, (C.c_size_t * 3)(N), (C.c_float * 3)(0.1))
+    st = lib.bitnet_bitlinear_forward_fused(4096, C.byref(stack), 4096, C.byref(glue), 4096, M, K, None, 1 << 20, 1 << 40, None)
+    assert st == getattr(L, status), lib.bitnet_last_error_string()

@@ -312,6 +312,14 @@ def test_ffn_of_any_width_in_smaller_workspaces(M, H, F):
         st = lib.bitnet_ffn_forward(wg.data_ptr(), 0.05, wu.data_ptr(), 0.04, wd.data_ptr(), 0.03, x.data_ptr(), h.data_ptr(), y.data_ptr(),
                                     M, H, F, None, base, nbytes, torch.cuda.current_stream().cuda_stream)
         assert st == 0 and torch.equal(h, rh) and torch.equal(y, ry), nbytes
+    # the generic kernel's workspace also takes buffers at any address
+    xs, ws2 = torch.empty(M * H + 4, device="cuda"), torch.empty(wg.numel() + 16, dtype=torch.uint8, device="cuda")
+    xs[1:1 + M * H] = x.view(-1)
+    ws2[1:1 + wg.numel()] = wg
+    y = torch.full_like(x, float("nan"))
+    st = lib.bitnet_ffn_forward(ws2.data_ptr() + 1, 0.05, wu.data_ptr(), 0.04, wd.data_ptr(), 0.03, xs.data_ptr() + 4, h.data_ptr(), y.data_ptr(),
+                                M, H, F, None, base, size[L.PATH_GENERIC], torch.cuda.current_stream().cuda_stream)
+    assert st == 0 and torch.equal(y, ry)
     assert ops.device_error_flags() == 0
 
 
