@@ -514,8 +514,8 @@ static bitnet_status_t ffn_impl(const uint8_t *w_gate_dev, float s_gate, const u
     // a block with a width that is no multiple of 128 makes do with less workspace: that projection, or else (also where buffers
     // are not aligned) all three, on the generic kernel
     int path = o.path;
-    const bool odd = workspace_bytes >= ffn_workspace(M, hidden, ffn, path, glue);
-    if (path == BITNET_PATH_AUTO && (hidden % 128 || ffn % 128) && !odd) {
+    const bool odd = (hidden % 128 == 0 && ffn % 128 == 0) || workspace_bytes >= ffn_workspace(M, hidden, ffn, path, glue);
+    if (path == BITNET_PATH_AUTO && !odd) {
         const uintptr_t all = reinterpret_cast<uintptr_t>(w_gate_dev) | reinterpret_cast<uintptr_t>(w_up_dev) | reinterpret_cast<uintptr_t>(w_down_dev) |
                               reinterpret_cast<uintptr_t>(x_dev) | reinterpret_cast<uintptr_t>(h_dev);
         if ((all & 15) || workspace_bytes < ffn_workspace(M, hidden, ffn, path, glue, false)) path = BITNET_PATH_GENERIC;
